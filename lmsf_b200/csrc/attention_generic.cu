@@ -40,13 +40,14 @@ struct GenericAttnArgs {
   int keep_first;                              // > 0 (with a window): the first keep_first keys of the request stay visible behind the window
   int sigmoid;                                 // 1: a key's weight is sigmoid(score), not normalised over the keys (no softmax)
   const float* head_bias;                      // [n_q_heads] or null: a number per query head added to every scaled score
+  int wide;                                    // rows of the cache can be read four values at a time
   const float* dist; int dist_n;               // [n_q_heads][dist_n] or null: the entry of (query position - key position), the last for larger ones, is added
 };
 
 // MAXD: the largest head size of a build (accumulators in registers)
 template <typename T, int MAXD>
 __global__ void __launch_bounds__(kWarps * 32) attention_generic_kernel(GenericAttnArgs a) {
-  __shared__ float qs[MAXD];
+  __shared__ __align__(16) float qs[MAXD];
   __shared__ float part_acc[kWarps][MAXD];
   __shared__ float part_m[kWarps], part_l[kWarps];
 
@@ -91,7 +92,20 @@ __global__ void __launch_bounds__(kWarps * 32) attention_generic_kernel(GenericA
         row = (long long)page * a.page_stride + head_off + (size_t)(key % a.block_size) * hd;
         const T* kr = (const T*)a.cache + row;
         float dot = 0.f;
-        for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], to_f32(kr[d]), dot);
+        if (a.wide) {   // the same sum in the same order, in a quarter of the loads: a lane's row is a line of its own
+#pragma unroll 8
+          for (int d = 0; d < hd; d += 4) {
+            float kv[4];
+            ld4(kr + d, kv);
+            const float4 qv = *reinterpret_cast<const float4*>(qs + d);
+            dot = fmaf(qv.x, kv[0], dot);
+            dot = fmaf(qv.y, kv[1], dot);
+            dot = fmaf(qv.z, kv[2], dot);
+            dot = fmaf(qv.w, kv[3], dot);
+          }
+        } else {
+          for (int d = 0; d < hd; ++d) dot = fmaf(qs[d], to_f32(kr[d]), dot);
+        }
         s = dot * a.scale;
         if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
         if (a.slopes) s = fmaf(a.slopes[head], (float)(key - pos), s);
@@ -122,15 +136,25 @@ __global__ void __launch_bounds__(kWarps * 32) attention_generic_kernel(GenericA
     l = l * alpha + warp_sum(p);
 #pragma unroll
     for (int i = 0; i < MAXD / 32; ++i) acc[i] *= alpha;
-    for (int j = 0; j < 32; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      const long long rj = __shfl_sync(0xffffffffu, row, j);
-      if (rj < 0) continue;  // same for the whole warp
-      const T* vr = (const T*)a.cache + rj + v_off;
+    // kVB values are asked for at a time; a key that is not seen has p = 0 and adds zero
+    constexpr int kVB = MAXD <= 128 ? 8 : 1;
+    for (int j0 = 0; j0 < 32; j0 += kVB) {
+      T v[kVB][MAXD / 32];
 #pragma unroll
-      for (int i = 0; i < MAXD / 32; ++i) {
-        const int d = lane + 32 * i;
-        if (i < nd && d < hd) acc[i] = fmaf(pj, to_f32(vr[d]), acc[i]);
+      for (int u = 0; u < kVB; ++u) {
+        const long long rj = __shfl_sync(0xffffffffu, row, j0 + u);
+        const T* vr = (const T*)a.cache + rj + v_off;
+#pragma unroll
+        for (int i = 0; i < MAXD / 32; ++i) {
+          const int d = lane + 32 * i;
+          v[u][i] = (rj >= 0 && i < nd && d < hd) ? vr[d] : from_f32<T>(0.f);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kVB; ++u) {
+        const float pj = __shfl_sync(0xffffffffu, p, j0 + u);
+#pragma unroll
+        for (int i = 0; i < MAXD / 32; ++i) acc[i] = fmaf(pj, to_f32(v[u][i]), acc[i]);
       }
     }
     m = m_new;
@@ -205,14 +229,16 @@ LMSF_API int lmsf_attention_generic_dist(const void* q, long long q_stride, void
   GenericAttnArgs a{q, q_stride, out, out_stride, cache, page_stride, block_table, max_blocks, block_size,
                     token_seq, positions, scale, window, n_q_heads, n_kv_heads, head_dim, softcap > 0.f ? softcap : 0.f, slopes,
                     shared_kv ? 1 : 0, gate, gate_stride, chunk > 0 ? chunk : 0, log_r1, log_r2, sinks,
-                    (window > 0 && keep_first > 0) ? keep_first : 0, sigmoid ? 1 : 0, head_bias, dist, dist_n};
+                    (window > 0 && keep_first > 0) ? keep_first : 0, sigmoid ? 1 : 0, head_bias,
+                    page_stride % 4 == 0 && (uintptr_t)cache % 16 == 0, dist, dist_n};
   if (dist && dist_n <= 0) LMSF_REFUSE("attention: a table of %d distances", dist_n);
   if (sigmoid && sinks) LMSF_REFUSE("attention: sinks belong to a softmax, not to sigmoid weights");
   dim3 grid(n_tokens, n_q_heads);
   cudaStream_t s = (cudaStream_t)stream;
 #define LMSF_GO(D) do { if (dtype == LMSF_F32) attention_generic_kernel<float, D><<<grid, kWarps * 32, 0, s>>>(a); \
                         else attention_generic_kernel<bf16, D><<<grid, kWarps * 32, 0, s>>>(a); } while (0)
-  if (head_dim <= 128) LMSF_GO(128);
+  if (head_dim <= 64) LMSF_GO(64);
+  else if (head_dim <= 128) LMSF_GO(128);
   else if (head_dim <= 256) LMSF_GO(256);
   else LMSF_GO(kMaxHeadDim);
 #undef LMSF_GO

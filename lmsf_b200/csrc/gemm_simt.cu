@@ -3,8 +3,12 @@
 // twin of the tensor-core products.  Counterpart in the reference: cublasLtMatmul through
 // tops/csrc/tops/tensorrt_llm/common/cublasMMWrapper.cpp:122-209.
 //
-// Every output element is accumulated by one thread over k = 0 .. K-1 in ascending order, so a
-// row's result does not depend on M or on which other rows share the launch.
+// Float32: K is cut into eight parts of part_len(K) values (a multiple of 32; the last ones may be empty).  A part's
+// products are added in ascending k by one chain of FMAs, and out = (((p0 + p1) + p2) + p3) + (((p4 + p5) + p6) + p7).
+// All three kernels below keep to that order, so a row's result does not depend by a bit on M, on which other rows share
+// the launch or on the kernel that was chosen.  (One chain over all of K, as before, leaves a product of few rows no
+// parallelism along k, and its rounding error is larger.)
+// bfloat16: every output element is accumulated by one thread over k = 0 .. K-1 in ascending order.
 #include "common.cuh"
 
 LMSF_DEFINE_LAST_ERROR(lmsf_gemm_simt)
@@ -13,6 +17,10 @@ namespace lmsf {
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
+constexpr int kParts = 8;
+__host__ __device__ constexpr int part_len(int K) { return ((K + kParts - 1) / kParts + 31) / 32 * 32; }
+
+// Any sizes and alignments, one scalar load per value.
 template <typename TA, typename TC>
 __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const TA* __restrict__ A,
                                                       const TA* __restrict__ W, int M, int N, int K, long long lda,
@@ -28,13 +36,26 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
   const int tx = tid % 16, ty = tid / 16;  // thread's 4x4 patch: rows ty*4.., cols tx*4..
   const int lr = tid / 4, lk = (tid % 4) * 4;  // loader: row lr of the tile, k offsets lk..lk+3
 
-  float acc[4][4];
+  float acc[4][4], tot[4][4], half[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = tot[i][j] = half[i][j] = 0.f;
+  const bool in_parts = sizeof(TA) == 4;   // float32: the sum of the parts
+  const int L = part_len(K);
 
   for (int k0 = 0; k0 < K; k0 += BK) {
+    if (in_parts && k0 > 0 && k0 % L == 0) {
+      const bool to_half = k0 == kParts / 2 * L;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          tot[i][j] += acc[i][j];
+          acc[i][j] = 0.f;
+          if (to_half) { half[i][j] = tot[i][j]; tot[i][j] = 0.f; }
+        }
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int k = k0 + lk + e;
@@ -64,9 +85,311 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      if (n < N) C[(size_t)m * ldc + n] = from_f32<TC>(acc[i][j]);
+      if (n < N) C[(size_t)m * ldc + n] = from_f32<TC>(in_parts ? half[i][j] + (tot[i][j] + acc[i][j]) : acc[i][j]);
     }
   }
+}
+
+// ---- float32, rows that can be read 16 bytes at a time ------------------------------------------------------
+
+struct F32Args {
+  float* C; const float* A; const float* W;
+  int M, N, K;
+  long long lda, ldw, ldc, batch_a, batch_w, batch_c;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {   // 16 bytes, zeros where there is nothing
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Up to 16 rows of A: a stream over W.  A block takes 16 rows of W, its warp w the parts 2 w (lanes 0..15, a row of W
+// each) and 2 w + 1 (lanes 16..31), through a ring of its own of cp.async stages of 32 k: 4 KB of W (chunks of 16 bytes
+// swizzled by the row, so that eight lanes read eight different banks) and the matching x, which all lanes of a part read
+// together.  Bound by the stream: with five stages (three at 16 rows) two blocks fit an SM and keep 128 KB of W asked for.  W's first stages
+// are asked for before the kernel before this one has ended.  At 3 rows, alone and
+// with a cold L2: 128,256 x 2,048 in 213 us (4.9 TB/s), 16,384 x 2,048 in 47 us, 2,048 x 8,192 in 35 us.  (Prompts of
+// 515 tokens and 12 decoded tokens for three requests, Llama-3.2-1B: 294 -> 55.8 ms with this kernel and the next.)
+template <int NT> constexpr int few_stages = NT <= 4 ? 5 : (NT == 8 ? 4 : 3);
+template <int NT>
+__global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
+  constexpr int kFewStages = few_stages<NT>;
+  constexpr int kStage = 4096 + 2 * NT * 128;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = lane & 15, h = lane >> 4;
+  const int n0 = blockIdx.x * 16;
+  const float* A = a.A + (size_t)blockIdx.y * a.batch_a;
+  const float* W = a.W + (size_t)blockIdx.y * a.batch_w;
+  float* C = a.C + (size_t)blockIdx.y * a.batch_c;
+  const int L = part_len(a.K), first = 2 * warp * L;
+  const int n_st = first < a.K ? L / 32 : 0;          // the second part's values beyond K are zeros
+  const uint32_t ring = smem_u32(smem) + warp * (kFewStages * kStage);
+
+  auto issue_w = [&](int c) {
+    const uint32_t st = ring + (c % kFewStages) * kStage;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int idx = lane + 32 * i, row = idx >> 3, ch = idx & 7;
+      const int k = first + (row >> 4) * L + c * 32 + ch * 4, n = n0 + (row & 15);
+      const bool ok = n < a.N && k < a.K;
+      cp16(st + row * 128 + ((ch ^ (row & 7)) << 4), ok ? W + (size_t)n * a.ldw + k : W, ok);
+    }
+  };
+  auto issue_x = [&](int c) {
+    const uint32_t st = ring + (c % kFewStages) * kStage + 4096;
+#pragma unroll
+    for (int i = 0; i < (NT * 16 + 31) / 32; ++i) {
+      const int idx = lane + 32 * i, row = idx >> 3, ch = idx & 7;
+      if (NT * 16 < 32 && row >= 2 * NT) break;
+      const int k = first + (row / NT) * L + c * 32 + ch * 4, m = row % NT;
+      const bool ok = m < a.M && k < a.K;
+      cp16(st + row * 128 + (ch << 4), ok ? A + (size_t)m * a.lda + k : A, ok);
+    }
+  };
+  pdl_launch_dependents();
+  for (int s = 0; s < kFewStages - 1; ++s)
+    if (s < n_st) issue_w(s);
+  pdl_wait();
+  for (int s = 0; s < kFewStages - 1; ++s) {
+    if (s < n_st) issue_x(s);
+    cp_commit();
+  }
+
+  float acc[NT];
+#pragma unroll
+  for (int m = 0; m < NT; ++m) acc[m] = 0.f;
+  for (int c = 0; c < n_st; ++c) {
+    cp_wait<kFewStages - 2>();
+    __syncwarp();
+    if (c + kFewStages - 1 < n_st) { issue_w(c + kFewStages - 1); issue_x(c + kFewStages - 1); }
+    cp_commit();
+    const unsigned char* st = smem + warp * (kFewStages * kStage) + (c % kFewStages) * kStage;
+    const unsigned char* xs = st + 4096 + h * (NT * 128);
+#pragma unroll(NT <= 8 ? 8 : 2)
+    for (int j = 0; j < 8; ++j) {
+      const float4 w = *reinterpret_cast<const float4*>(st + lane * 128 + ((j ^ (r & 7)) << 4));
+#pragma unroll
+      for (int m = 0; m < NT; ++m) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + m * 128 + (j << 4));
+        acc[m] = fmaf(x.x, w.x, acc[m]);
+        acc[m] = fmaf(x.y, w.y, acc[m]);
+        acc[m] = fmaf(x.z, w.z, acc[m]);
+        acc[m] = fmaf(x.w, w.w, acc[m]);
+      }
+    }
+  }
+  cp_wait<0>();
+  __syncthreads();
+  float* part = reinterpret_cast<float*>(smem);       // [part][m][row]
+#pragma unroll
+  for (int m = 0; m < NT; ++m) part[((2 * warp + h) * NT + m) * 16 + r] = acc[m];
+  __syncthreads();
+  for (int i = threadIdx.x; i < NT * 16; i += 128) {
+    const int m = i / 16, n = n0 + i % 16;
+    if (m >= a.M || n >= a.N) continue;
+    float p[kParts];
+#pragma unroll
+    for (int q = 0; q < kParts; ++q) p[q] = part[q * NT * 16 + i];
+    C[(size_t)m * a.ldc + n] = (((p[0] + p[1]) + p[2]) + p[3]) + (((p[4] + p[5]) + p[6]) + p[7]);
+  }
+}
+
+// More rows: tiles of 64 rows of A and 128 of W by 128 threads with 8 x 8 results each (a row of A every 8 rows, a row of W
+// every 16, so that the reads of four k of a warp's 4 x 8 lanes fall on different banks), cp.async stages of 32 k.  Bound by the
+// FMA pipe; 256 FMAs per 16 reads of 16 bytes.  CS: blocks of a cluster that share a tile along k, where the tiles alone
+// leave SMs idle: 2 (a half of the parts each) or 8 (a part each); their sums meet in shared memory.  At 515 rows
+// 16,384 x 2,048 takes 1.00 ms (34.6 TFLOP/s), 2,048 x 8,192 0.50 ms, 2,048 x 2,048 0.145 ms.
+constexpr int TM = 64, TN = 128, TK = 32, kTileStages = 3, kTileRow = TK * 4 + 16, kTileStage = (TM + TN) * kTileRow;
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_remote(uint32_t addr, int rank) {
+  uint32_t ra;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+  return v;
+}
+
+template <int CS>
+__global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = blockIdx.x % CS;                    // clusters lie along x
+  const int m0 = blockIdx.x / CS * TM, n0 = blockIdx.y * TN;
+  const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);   // rows tx + 16 j of W, ty + 8 i of A
+  const float* A = a.A + (size_t)blockIdx.z * a.batch_a;
+  const float* W = a.W + (size_t)blockIdx.z * a.batch_w;
+  float* C = a.C + (size_t)blockIdx.z * a.batch_c;
+  const int L = part_len(a.K), first = rank * (kParts / CS) * L, st_part = L / TK;
+  const int n_st = first < a.K ? min(kParts / CS * st_part, (a.K - first + TK - 1) / TK) : 0;
+  const uint32_t base = smem_u32(smem);
+
+  auto issue = [&](int s) {
+    const uint32_t st = base + (s % kTileStages) * kTileStage;
+    const int k0 = first + s * TK;
+#pragma unroll
+    for (int i = 0; i < (TM + TN) * 8 / 128; ++i) {
+      const int idx = tid + 128 * i, row = idx >> 3, ch = idx & 7, k = k0 + ch * 4;
+      const bool of_a = row < TM;                      // the same for all threads of a pass
+      const int g = of_a ? m0 + row : n0 + row - TM;
+      const bool ok = g < (of_a ? a.M : a.N) && k < a.K;
+      const float* src = of_a ? A + (size_t)g * a.lda + k : W + (size_t)g * a.ldw + k;
+      cp16(st + row * kTileRow + (ch << 4), ok ? src : a.A, ok);
+    }
+  };
+
+  float acc[8][8], tot[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = tot[i][j] = 0.f;
+  for (int s = 0; s < kTileStages - 1; ++s) {
+    if (s < n_st) issue(s);
+    cp_commit();
+  }
+  bool parked = false;                                 // CS 1: the first four parts' sum waits in C
+  int next_fold = st_part;
+  for (int s = 0; s < n_st; ++s) {
+    cp_wait<kTileStages - 2>();
+    __syncthreads();
+    if (s + kTileStages - 1 < n_st) issue(s + kTileStages - 1);
+    cp_commit();
+    const unsigned char* st = smem + (s % kTileStages) * kTileStage;
+    const unsigned char* as = st + ty * kTileRow;
+    const unsigned char* ws = st + (TM + tx) * kTileRow;
+#pragma unroll
+    for (int k4 = 0; k4 < TK / 4; ++k4) {
+      float4 w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(ws + 16 * j * kTileRow + k4 * 16);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(as + 8 * i * kTileRow + k4 * 16);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.x, w[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.y, w[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.z, w[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.w, w[j].w, acc[i][j]);
+      }
+    }
+    if (CS < kParts && s + 1 == next_fold) {
+      next_fold += st_part;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { tot[i][j] += acc[i][j]; acc[i][j] = 0.f; }
+      if (CS == 1 && s + 1 == kParts / 2 * st_part && s + 1 < n_st) {
+        parked = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
+            if (m < a.M && n < a.N) C[(size_t)m * a.ldc + n] = tot[i][j];
+            tot[i][j] = 0.f;
+          }
+      }
+    }
+  }
+  cp_wait<0>();
+  if (CS < kParts) {                                   // a last part that K cuts short (nothing is left else)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) tot[i][j] += acc[i][j];
+  }
+  if constexpr (CS == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
+        if (m < a.M && n < a.N) {
+          float* c = C + (size_t)m * a.ldc + n;
+          *c = parked ? *c + tot[i][j] : tot[i][j];
+        }
+      }
+  } else {
+    __syncthreads();                                   // every warp has read its last stage
+    float* mine = reinterpret_cast<float*>(smem);      // [8 i + j][thread]
+    if (CS == kParts || rank == 1) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mine[(8 * i + j) * 128 + tid] = CS == kParts ? acc[i][j] : tot[i][j];
+    }
+    cluster_sync();
+    if (CS == 2 && rank == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
+          const float v = tot[i][j] + ld_remote(base + ((8 * i + j) * 128 + tid) * 4, 1);
+          if (m < a.M && n < a.N) C[(size_t)m * a.ldc + n] = v;
+        }
+    }
+    if (CS == kParts) {                                // block `rank` adds up the rows ty + 8 rank of the tile
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float p[kParts];
+#pragma unroll
+        for (int q = 0; q < kParts; ++q) p[q] = ld_remote(base + ((8 * rank + j) * 128 + tid) * 4, q);
+        const int m = m0 + ty + 8 * rank, n = n0 + tx + 16 * j;
+        if (m < a.M && n < a.N)
+          C[(size_t)m * a.ldc + n] = (((p[0] + p[1]) + p[2]) + p[3]) + (((p[4] + p[5]) + p[6]) + p[7]);
+      }
+    }
+    cluster_sync();                                    // nobody leaves while its sums are being read
+  }
+}
+
+template <int NT>
+static int launch_few_rows(const F32Args& a, int batch, cudaStream_t s) {
+  constexpr int smem = 4 * few_stages<NT> * (4096 + 2 * NT * 128);
+  cudaError_t e = cudaFuncSetAttribute(f32_few_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  return launch_pdl(f32_few_rows_kernel<NT>, dim3(ceil_div(a.N, 16), batch), dim3(128), smem, s, a);
+}
+
+template <int CS>
+static int launch_tile(const F32Args& a, int batch, cudaStream_t s) {
+  constexpr int smem = kTileStages * kTileStage;
+  cudaError_t e = cudaFuncSetAttribute(f32_tile_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div(a.M, TM) * CS, ceil_div(a.N, TN), batch);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, f32_tile_kernel<CS>, a);
+}
+
+static int launch_f32(const F32Args& a, int batch, cudaStream_t s) {
+  if (a.M <= 1) return launch_few_rows<1>(a, batch, s);
+  if (a.M <= 2) return launch_few_rows<2>(a, batch, s);
+  if (a.M <= 4) return launch_few_rows<4>(a, batch, s);
+  if (a.M <= 8) return launch_few_rows<8>(a, batch, s);
+  if (a.M <= 16) return launch_few_rows<16>(a, batch, s);
+  // two blocks fit an SM: the tiles alone where they fill the device, else shared along k
+  const long long tiles = (long long)ceil_div(a.M, TM) * ceil_div(a.N, TN) * batch;
+  if (tiles >= 296) return launch_tile<1>(a, batch, s);
+  if (tiles >= 74) return launch_tile<2>(a, batch, s);
+  return launch_tile<8>(a, batch, s);
 }
 
 }  // namespace lmsf
@@ -85,6 +408,10 @@ LMSF_API int lmsf_gemm_tn_simt_batched(void* C, const void* A, const void* W, in
   dim3 grid(ceil_div(N, BN), ceil_div(M, BM), batch);
   if (grid.y > 65535) LMSF_REFUSE("gemm: M=%d is too large for one launch", M);
   cudaStream_t s = (cudaStream_t)stream;
+  const bool wide = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && batch_a % 4 == 0 && batch_w % 4 == 0 &&
+                    (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+  if (in_dtype == LMSF_F32 && out_dtype == LMSF_F32 && wide && ceil_div(N, TN) <= 65535)
+    return launch_f32(F32Args{(float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c}, batch, s);
   if (in_dtype == LMSF_F32 && out_dtype == LMSF_F32)
     gemm_tn_kernel<float, float><<<grid, 256, 0, s>>>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
   else if (in_dtype == LMSF_BF16 && out_dtype == LMSF_BF16)

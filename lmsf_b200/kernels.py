@@ -424,7 +424,8 @@ def bias_add(x: torch.Tensor, bias: torch.Tensor):
 # ----------------------------------------------------------------------------- SIMT matrix product
 
 def gemm_tn_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
-    """out[M, N] = a[M, K] w[N, K]^T, float32 FMA accumulation in ascending k (true 32-bit when a, w are float32)."""
+    """out[M, N] = a[M, K] w[N, K]^T, float32 FMA accumulation in a fixed order, whatever M is (true 32-bit when
+    a, w are float32: eight sums over ascending k, added up)."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N) or a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
@@ -1461,7 +1462,7 @@ def attention_shared_kv(out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor,
 
 def gemm_tn_simt_batched(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
     """out[:, b, :] = a[:, b, :] w[b]^T for every b.  a: [M, B, K], out: [M, B, N] (views: the last dimension
-    contiguous, any row and batch strides); w: [B, N, K].  float32 FMA accumulation in ascending k."""
+    contiguous, any row and batch strides); w: [B, N, K].  float32 FMA accumulation in the order of `gemm_tn_simt`."""
     M, B, K = a.shape
     N = w.shape[1]
     if w.shape != (B, N, K) or out.shape != (M, B, N) or a.stride(2) != 1 or w.stride(2) != 1 or out.stride(2) != 1 \
