@@ -3,8 +3,9 @@
 // twin of the tensor-core products.  Counterpart in the reference: cublasLtMatmul through
 // tops/csrc/tops/tensorrt_llm/common/cublasMMWrapper.cpp:122-209.
 //
-// Float32: K is cut into eight parts of part_len(K) values (a multiple of 32; the last ones may be empty).  A part's
-// products are added in ascending k by one chain of FMAs, and out = (((p0 + p1) + p2) + p3) + (((p4 + p5) + p6) + p7).
+// Float32: K is cut into eight parts of part_len(K) values (a multiple of 32; the last ones may be empty).  A part is the
+// sum of two chains of FMAs in ascending k, of its even k and of its odd k (the two halves of fma.rn.f32x2 on the values as
+// they lie in memory), and out = (((p0 + p1) + p2) + p3) + (((p4 + p5) + p6) + p7).
 // All three kernels below keep to that order, so a row's result does not depend by a bit on M, on which other rows share
 // the launch or on the kernel that was chosen.  (One chain over all of K, as before, leaves a product of few rows no
 // parallelism along k, and its rounding error is larger.)
@@ -36,11 +37,11 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
   const int tx = tid % 16, ty = tid / 16;  // thread's 4x4 patch: rows ty*4.., cols tx*4..
   const int lr = tid / 4, lk = (tid % 4) * 4;  // loader: row lr of the tile, k offsets lk..lk+3
 
-  float acc[4][4], tot[4][4], half[4][4];
+  float acc[4][4], odd[4][4], tot[4][4], half[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = tot[i][j] = half[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = odd[i][j] = tot[i][j] = half[i][j] = 0.f;
   const bool in_parts = sizeof(TA) == 4;   // float32: the sum of the parts
   const int L = part_len(K);
 
@@ -51,8 +52,8 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          tot[i][j] += acc[i][j];
-          acc[i][j] = 0.f;
+          tot[i][j] += acc[i][j] + odd[i][j];
+          acc[i][j] = odd[i][j] = 0.f;
           if (to_half) { half[i][j] = tot[i][j]; tot[i][j] = 0.f; }
         }
     }
@@ -74,7 +75,10 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) {
+          float& c = in_parts && (kk & 1) ? odd[i][j] : acc[i][j];
+          c = fmaf(a[i], w[j], c);
+        }
     }
     __syncthreads();
   }
@@ -85,7 +89,7 @@ __global__ void __launch_bounds__(256) gemm_tn_kernel(TC* __restrict__ C, const 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
-      if (n < N) C[(size_t)m * ldc + n] = from_f32<TC>(in_parts ? half[i][j] + (tot[i][j] + acc[i][j]) : acc[i][j]);
+      if (n < N) C[(size_t)m * ldc + n] = from_f32<TC>(in_parts ? half[i][j] + (tot[i][j] + (acc[i][j] + odd[i][j])) : acc[i][j]);
     }
   }
 }
@@ -102,6 +106,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {   // 16 bytes, zeros where there is nothing
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// d += a * b, both halves
+__device__ __forceinline__ void fma2(float2& d, float ax, float ay, float bx, float by) {
+  asm("{\n.reg .b64 a, b, c;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%0, %1};\nfma.rn.f32x2 c, a, b, c;\nmov.b64 {%0, %1}, c;\n}\n"
+      : "+f"(d.x), "+f"(d.y) : "f"(ax), "f"(ay), "f"(bx), "f"(by));
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -109,13 +121,14 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // each) and 2 w + 1 (lanes 16..31), through a ring of its own of cp.async stages of 32 k: 4 KB of W (chunks of 16 bytes
 // swizzled by the row, so that eight lanes read eight different banks) and the matching x, which all lanes of a part read
 // together.  Bound by the stream: with five stages (three at 16 rows) two blocks fit an SM and keep 128 KB of W asked for.  W's first stages
-// are asked for before the kernel before this one has ended.  At 3 rows, alone and
-// with a cold L2: 128,256 x 2,048 in 213 us (4.9 TB/s), 16,384 x 2,048 in 47 us, 2,048 x 8,192 in 35 us.  (Prompts of
-// 515 tokens and 12 decoded tokens for three requests, Llama-3.2-1B: 294 -> 55.8 ms with this kernel and the next.)
-template <int NT> constexpr int few_stages = NT <= 4 ? 5 : (NT == 8 ? 4 : 3);
-template <int NT>
+// are asked for before the kernel before this one has ended.  One launch after the
+// other on different weights at 3 rows: 128,256 x 2,048 in 151 us (7.0 TB/s), 16,384 x 2,048 in 25 us (5.3), 2,048 x 8,192 in
+// 14 us (4.8); 31 and 25 us for the last two with single FMAs and an address per copy.  (Prompts of 515 tokens and 12 decoded
+// tokens for three requests, Llama-3.2-1B: 294 -> 50.8 ms with this kernel and the next.)
+template <int NT, bool DEEP> constexpr int few_stages = (NT <= 4 ? 5 : (NT <= 8 ? 4 : 3)) * (DEEP ? 2 : 1);
+template <int NT, bool DEEP>
 __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
-  constexpr int kFewStages = few_stages<NT>;
+  constexpr int kFewStages = few_stages<NT, DEEP>;
   constexpr int kStage = 4096 + 2 * NT * 128;
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -128,22 +141,32 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
   const int n_st = first < a.K ? L / 32 : 0;          // the second part's values beyond K are zeros
   const uint32_t ring = smem_u32(smem) + warp * (kFewStages * kStage);
 
+  // the lane's copies: chunk ch of rows r0, r0 + 4, ... of the first part, then of the second
+  const int r0 = lane >> 3, ch = lane & 7;
+  const float* w0 = W + (size_t)(n0 + r0) * a.ldw + first + ch * 4;
+  const size_t w_step = (size_t)4 * a.ldw;
+  const bool whole = n0 + 16 <= a.N && a.K == kParts * L;        // nothing to leave out
   auto issue_w = [&](int c) {
     const uint32_t st = ring + (c % kFewStages) * kStage;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int idx = lane + 32 * i, row = idx >> 3, ch = idx & 7;
-      const int k = first + (row >> 4) * L + c * 32 + ch * 4, n = n0 + (row & 15);
-      const bool ok = n < a.N && k < a.K;
-      cp16(st + row * 128 + ((ch ^ (row & 7)) << 4), ok ? W + (size_t)n * a.ldw + k : W, ok);
+      const int row = r0 + 4 * i;
+      const uint32_t dst = st + row * 128 + ((ch ^ (row & 7)) << 4);
+      const float* src = w0 + (i & 3) * w_step + (i >> 2) * L + c * 32;
+      if (whole) {
+        cp16(dst, src);
+      } else {
+        const bool ok = n0 + (row & 15) < a.N && first + (i >> 2) * L + c * 32 + ch * 4 < a.K;
+        cp16(dst, ok ? src : W, ok);
+      }
     }
   };
   auto issue_x = [&](int c) {
     const uint32_t st = ring + (c % kFewStages) * kStage + 4096;
 #pragma unroll
     for (int i = 0; i < (NT * 16 + 31) / 32; ++i) {
-      const int idx = lane + 32 * i, row = idx >> 3, ch = idx & 7;
-      if (NT * 16 < 32 && row >= 2 * NT) break;
+      const int row = r0 + 4 * i;
+      if (NT % 2 && row >= 2 * NT) break;
       const int k = first + (row / NT) * L + c * 32 + ch * 4, m = row % NT;
       const bool ok = m < a.M && k < a.K;
       cp16(st + row * 128 + (ch << 4), ok ? A + (size_t)m * a.lda + k : A, ok);
@@ -158,9 +181,9 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
     cp_commit();
   }
 
-  float acc[NT];
+  float2 acc[NT];
 #pragma unroll
-  for (int m = 0; m < NT; ++m) acc[m] = 0.f;
+  for (int m = 0; m < NT; ++m) acc[m] = make_float2(0.f, 0.f);
   for (int c = 0; c < n_st; ++c) {
     cp_wait<kFewStages - 2>();
     __syncwarp();
@@ -174,10 +197,8 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
 #pragma unroll
       for (int m = 0; m < NT; ++m) {
         const float4 x = *reinterpret_cast<const float4*>(xs + m * 128 + (j << 4));
-        acc[m] = fmaf(x.x, w.x, acc[m]);
-        acc[m] = fmaf(x.y, w.y, acc[m]);
-        acc[m] = fmaf(x.z, w.z, acc[m]);
-        acc[m] = fmaf(x.w, w.w, acc[m]);
+        fma2(acc[m], x.x, x.y, w.x, w.y);
+        fma2(acc[m], x.z, x.w, w.z, w.w);
       }
     }
   }
@@ -185,7 +206,7 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
   __syncthreads();
   float* part = reinterpret_cast<float*>(smem);       // [part][m][row]
 #pragma unroll
-  for (int m = 0; m < NT; ++m) part[((2 * warp + h) * NT + m) * 16 + r] = acc[m];
+  for (int m = 0; m < NT; ++m) part[((2 * warp + h) * NT + m) * 16 + r] = acc[m].x + acc[m].y;
   __syncthreads();
   for (int i = threadIdx.x; i < NT * 16; i += 128) {
     const int m = i / 16, n = n0 + i % 16;
@@ -199,10 +220,11 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
 
 // More rows: tiles of 64 rows of A and 128 of W by 128 threads with 8 x 8 results each (a row of A every 8 rows, a row of W
 // every 16, so that the reads of four k of a warp's 4 x 8 lanes fall on different banks), cp.async stages of 32 k.  Bound by the
-// FMA pipe; 256 FMAs per 16 reads of 16 bytes.  CS: blocks of a cluster that share a tile along k, where the tiles alone
+// FMA pipe; 128 fma.rn.f32x2 per 16 reads of 16 bytes (single FMAs stalled on their operands' register banks).  CS: blocks of a cluster that share a tile along k, where the tiles alone
 // leave SMs idle: 2 (a half of the parts each) or 8 (a part each); their sums meet in shared memory.  At 515 rows
-// 16,384 x 2,048 takes 1.00 ms (34.6 TFLOP/s), 2,048 x 8,192 0.50 ms, 2,048 x 2,048 0.145 ms.
-constexpr int TM = 64, TN = 128, TK = 32, kTileStages = 3, kTileRow = TK * 4 + 16, kTileStage = (TM + TN) * kTileRow;
+// 16,384 x 2,048 takes 0.87 ms (39.6 TFLOP/s), 2,048 x 8,192 0.45 ms, 2,048 x 2,048 0.122 ms; 0.99, 0.49 and 0.131 ms with
+// single FMAs.
+constexpr int TM = 64, TN = 128, TK = 32, kTileStages = 2, kTileRow = TK * 4 + 16, kTileStage = (TM + TN) * kTileRow;
 
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -243,17 +265,18 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
     }
   };
 
-  float acc[8][8], tot[8][8];
+  float2 acc[8][8];
+  float* tot = reinterpret_cast<float*>(smem + kTileStages * kTileStage);   // [8 i + j][thread]: the parts of a half so far
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = tot[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
   for (int s = 0; s < kTileStages - 1; ++s) {
     if (s < n_st) issue(s);
     cp_commit();
   }
   bool parked = false;                                 // CS 1: the first four parts' sum waits in C
-  int next_fold = st_part;
+  int next_fold = st_part, parts_in_half = 0;
   for (int s = 0; s < n_st; ++s) {
     cp_wait<kTileStages - 2>();
     __syncthreads();
@@ -271,41 +294,37 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
       for (int i = 0; i < 8; ++i) {
         const float4 x = *reinterpret_cast<const float4*>(as + 8 * i * kTileRow + k4 * 16);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.x, w[j].x, acc[i][j]);
+        for (int j = 0; j < 8; ++j) fma2(acc[i][j], x.x, x.y, w[j].x, w[j].y);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.y, w[j].y, acc[i][j]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.z, w[j].z, acc[i][j]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x.w, w[j].w, acc[i][j]);
+        for (int j = 0; j < 8; ++j) fma2(acc[i][j], x.z, x.w, w[j].z, w[j].w);
       }
     }
-    if (CS < kParts && s + 1 == next_fold) {
+    if (CS < kParts && (s + 1 == next_fold || s + 1 == n_st)) {
       next_fold += st_part;
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { tot[i][j] += acc[i][j]; acc[i][j] = 0.f; }
+        for (int j = 0; j < 8; ++j) {
+          float* t = tot + (8 * i + j) * 128 + tid;
+          const float p = acc[i][j].x + acc[i][j].y;
+          *t = parts_in_half ? *t + p : p;
+          acc[i][j] = make_float2(0.f, 0.f);
+        }
+      ++parts_in_half;
       if (CS == 1 && s + 1 == kParts / 2 * st_part && s + 1 < n_st) {
         parked = true;
+        parts_in_half = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
-            if (m < a.M && n < a.N) C[(size_t)m * a.ldc + n] = tot[i][j];
-            tot[i][j] = 0.f;
+            if (m < a.M && n < a.N) C[(size_t)m * a.ldc + n] = tot[(8 * i + j) * 128 + tid];
           }
       }
     }
   }
   cp_wait<0>();
-  if (CS < kParts) {                                   // a last part that K cuts short (nothing is left else)
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) tot[i][j] += acc[i][j];
-  }
   if constexpr (CS == 1) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -314,17 +333,17 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
         const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
         if (m < a.M && n < a.N) {
           float* c = C + (size_t)m * a.ldc + n;
-          *c = parked ? *c + tot[i][j] : tot[i][j];
+          const float t = tot[(8 * i + j) * 128 + tid];
+          *c = parked ? *c + t : t;
         }
       }
   } else {
-    __syncthreads();                                   // every warp has read its last stage
-    float* mine = reinterpret_cast<float*>(smem);      // [8 i + j][thread]
-    if (CS == kParts || rank == 1) {
+    const uint32_t tot_addr = base + kTileStages * kTileStage;
+    if (CS == kParts || parts_in_half == 0) {          // a part each, or a half that K does not reach (zeros)
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) mine[(8 * i + j) * 128 + tid] = CS == kParts ? acc[i][j] : tot[i][j];
+        for (int j = 0; j < 8; ++j) tot[(8 * i + j) * 128 + tid] = acc[i][j].x + acc[i][j].y;
     }
     cluster_sync();
     if (CS == 2 && rank == 0) {
@@ -333,7 +352,7 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int m = m0 + ty + 8 * i, n = n0 + tx + 16 * j;
-          const float v = tot[i][j] + ld_remote(base + ((8 * i + j) * 128 + tid) * 4, 1);
+          const float v = tot[(8 * i + j) * 128 + tid] + ld_remote(tot_addr + ((8 * i + j) * 128 + tid) * 4, 1);
           if (m < a.M && n < a.N) C[(size_t)m * a.ldc + n] = v;
         }
     }
@@ -342,7 +361,7 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
       for (int j = 0; j < 8; ++j) {
         float p[kParts];
 #pragma unroll
-        for (int q = 0; q < kParts; ++q) p[q] = ld_remote(base + ((8 * rank + j) * 128 + tid) * 4, q);
+        for (int q = 0; q < kParts; ++q) p[q] = ld_remote(tot_addr + ((8 * rank + j) * 128 + tid) * 4, q);
         const int m = m0 + ty + 8 * rank, n = n0 + tx + 16 * j;
         if (m < a.M && n < a.N)
           C[(size_t)m * a.ldc + n] = (((p[0] + p[1]) + p[2]) + p[3]) + (((p[4] + p[5]) + p[6]) + p[7]);
@@ -352,17 +371,35 @@ __global__ void __launch_bounds__(128, 2) f32_tile_kernel(F32Args a) {
   }
 }
 
+static int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  }
+  return n;
+}
+
+template <int NT, bool DEEP>
+static int launch_few(const F32Args& a, int batch, cudaStream_t s) {
+  constexpr int smem = 4 * few_stages<NT, DEEP> * (4096 + 2 * NT * 128);
+  cudaError_t e = cudaFuncSetAttribute(f32_few_rows_kernel<NT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  return launch_pdl(f32_few_rows_kernel<NT, DEEP>, dim3(ceil_div(a.N, 16), batch), dim3(128), smem, s, a);
+}
+
+// At most one block an SM and a long stream each (K of 4,096 and more): the ring takes all of the shared memory.
+// Shorter streams leave room for the next product's blocks, whose first stages then overlap.  (2,048 x 8,192 at 3
+// rows 17.0 -> 14.1 us.)
 template <int NT>
 static int launch_few_rows(const F32Args& a, int batch, cudaStream_t s) {
-  constexpr int smem = 4 * few_stages<NT> * (4096 + 2 * NT * 128);
-  cudaError_t e = cudaFuncSetAttribute(f32_few_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
-  return launch_pdl(f32_few_rows_kernel<NT>, dim3(ceil_div(a.N, 16), batch), dim3(128), smem, s, a);
+  const bool deep = (long long)ceil_div(a.N, 16) * batch <= sm_count() && a.K >= 4096;
+  return deep ? launch_few<NT, true>(a, batch, s) : launch_few<NT, false>(a, batch, s);
 }
 
 template <int CS>
 static int launch_tile(const F32Args& a, int batch, cudaStream_t s) {
-  constexpr int smem = kTileStages * kTileStage;
+  constexpr int smem = kTileStages * kTileStage + 64 * 128 * 4;
   cudaError_t e = cudaFuncSetAttribute(f32_tile_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
@@ -382,7 +419,9 @@ static int launch_tile(const F32Args& a, int batch, cudaStream_t s) {
 static int launch_f32(const F32Args& a, int batch, cudaStream_t s) {
   if (a.M <= 1) return launch_few_rows<1>(a, batch, s);
   if (a.M <= 2) return launch_few_rows<2>(a, batch, s);
+  if (a.M == 3) return launch_few_rows<3>(a, batch, s);
   if (a.M <= 4) return launch_few_rows<4>(a, batch, s);
+  if (a.M <= 6) return launch_few_rows<6>(a, batch, s);
   if (a.M <= 8) return launch_few_rows<8>(a, batch, s);
   if (a.M <= 16) return launch_few_rows<16>(a, batch, s);
   // two blocks fit an SM: the tiles alone where they fill the device, else shared along k

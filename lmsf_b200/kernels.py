@@ -425,7 +425,7 @@ def bias_add(x: torch.Tensor, bias: torch.Tensor):
 
 def gemm_tn_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
     """out[M, N] = a[M, K] w[N, K]^T, float32 FMA accumulation in a fixed order, whatever M is (true 32-bit when
-    a, w are float32: eight sums over ascending k, added up)."""
+    a, w are float32: sixteen sums over ascending k, added up)."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N) or a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:

@@ -145,7 +145,9 @@ class NormedParallelMixers(Mixer):
         self._in = torch.cat([L.qkv, R.in_proj, L.qkv.new_zeros((pad, L.qkv.shape[1]))], 0).contiguous()
         self._in_bias = None
         if L.qkv_bias is not None:
-            self._in_bias = torch.cat([L.qkv_bias, L.qkv_bias.new_zeros(rows + pad - n)], 0).contiguous()
+            # of the weights' type: the products add it to their float32 sums (a bias of another type is converted and added by
+            # kernels of their own in every step)
+            self._in_bias = torch.cat([L.qkv_bias, L.qkv_bias.new_zeros(rows + pad - n)], 0).to(self._in.dtype).contiguous()
         L.qkv, R.in_proj = self._in[:n], self._in[n:rows]  # the parts' own matrices become views of the merged one
 
     def forward(self, ctx: StepContext, h: torch.Tensor, cache: LayerCache) -> BranchPair:

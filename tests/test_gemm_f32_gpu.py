@@ -15,17 +15,18 @@ def _product(a, w):
     return out
 
 
-@pytest.mark.parametrize("N,K", [(1, 4), (15, 32), (129, 36), (300, 260), (128, 1024), (2048, 516), (257, 2052), (40000, 64)])
+@pytest.mark.parametrize("N,K", [(1, 4), (15, 32), (129, 36), (300, 260), (128, 1024), (2048, 516), (257, 2052), (64, 4096), (33, 4612), (40000, 64)])
 def test_every_route_gives_the_same_bits(N, K):
     g = torch.Generator(device="cuda").manual_seed(N + K)
     a = torch.randn(700, K, device="cuda", generator=g)
     w = torch.randn(N, K, device="cuda", generator=g)
     exact = a.double() @ w.double().T
-    # a chain of n FMAs errs by at most n 2^-24 times the sum of the products' sizes, here of K / 8 terms and eight parts
+    # a chain of n FMAs errs by at most n 2^-24 times the sum of the products' sizes; here no sum has passed through more than
+    # K / 16 + 16 FMAs of a chain, its other half and eight parts, and K / 8 + 40 is more
     bound = (math.ceil(K / 8) + 32 + 8) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
     whole = _product(a, w)
     assert bool(((whole.double() - exact).abs() <= bound).all())
-    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 64, 65, 128, 129, 500):
+    for m in (1, 2, 3, 4, 5, 6, 7, 8, 9, 16, 17, 64, 65, 128, 129, 500):
         assert torch.equal(_product(a[-m:], w), whole[-m:]), m
     # rows that cannot be read 16 bytes at a time
     odd_w = torch.empty(N, K + 1, device="cuda")[:, :K].copy_(w)
