@@ -277,8 +277,19 @@ class ModelRunner:
             bucket = self.graph_context_bucket(max(lens))
             skew = self.graph_skew_class(bucket, sum(lens) / len(lens))
         # a graph's block tables are as wide as its bucket of context lengths needs, not as the longest context allowed
-        hb = self._prepare(entries, mgr, (bucket + self.block_size - 1) // self.block_size if graph_mode else None,
+        batch, places = entries, None
+        if skew and len(entries) > 1:
+            # Requests of unequal length are laid out longest first, so that the decode attention starts with its longest blocks and
+            # the short ones fill its last wave; the rows whose logits are wanted keep the order of the
+            # entries.  (Contexts of 130 to 2,300 tokens: 64 requests of the 1B shape 1,660 -> 1,513 us a step, 27 of the 8B
+            # shape 4,677 -> 4,394.)
+            places = sorted(range(len(entries)), key=lambda i: -lens[i])
+            batch = [entries[i] for i in places]
+        hb = self._prepare(batch, mgr, (bucket + self.block_size - 1) // self.block_size if graph_mode else None,
                            self.graph_batch_size(len(entries)) if graph_mode else 0)
+        if places is not None:
+            rows = hb.pinned.numpy()[hb.seg["rows"][0]:]
+            rows[places] = np.arange(len(places), dtype=np.int32)
         self.storage.zero_state_slots(mgr.take_fresh_slots())
         key = (hb.S, bucket, skew) if graph_mode else None
         if graph_mode and (key in self._graphs or key in self._seen_sizes):
