@@ -218,10 +218,12 @@ class ModelRunner:
     # ------------------------------------------------------------------ the step
     @staticmethod
     def graph_batch_size(n: int) -> int:
-        """Decode batches are replayed from graphs of these sizes: 1, 2, 4, then multiples of 4 up to 32 (where the
+        """Decode batches are replayed from graphs of these sizes: 1 to 8, multiples of 4 up to 32 (where the
         decode attention's plan changes within a few requests: 20 requests take 4.4 ms a step on their own graph and
-        4.7 ms padded to 24), then multiples of 8."""
-        if n <= 2:
+        4.7 ms padded to 24), then multiples of 8.  (Few requests, above all of many kv heads, cannot afford stand-ins: 5
+        requests of the 13B shape at 3,900 keys took 8.81 ms a step padded to 8 and take 8.20, because the plan of the attention's splits counted
+        320 pairs of request and head where 200 have keys.)"""
+        if n <= 8:
             return n
         if n <= 32:
             return (n + 3) // 4 * 4
@@ -251,6 +253,19 @@ class ModelRunner:
         return (not self.enforce_eager and self.graph_safe and len(entries) <= self.max_graph_batch
                 and all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries))
 
+    @staticmethod
+    def _longest_first(entries: Sequence[StepEntry], mgr: CacheManager, lens: Optional[List[int]], skew: int) -> Optional[List[int]]:
+        """The order in which a step's entries are laid out, or None: as they come.  A replayed step is ordered where its
+        graph's class says so; another one where its single tokens' contexts differ (the longest is a third above the mean)."""
+        if lens is None:
+            lens = [mgr.num_tokens(e.request_id) + 1 if len(e.tokens) == 1 else 0 for e in entries]
+            decoding = [n for n in lens if n]
+            if len(decoding) < 2 or len(set(e.request_id for e in entries)) < len(entries) or 3 * max(decoding) * len(decoding) <= 4 * sum(decoding):
+                return None
+        elif not skew or len(entries) < 2:
+            return None
+        return sorted(range(len(entries)), key=lambda i: -lens[i])
+
     def _patch(self, hb: "_HostBatch", dev: torch.Tensor, pending_tokens: Optional[torch.Tensor]) -> None:
         if not hb.has_patches:
             return
@@ -266,7 +281,7 @@ class ModelRunner:
         of the entries and of their `want`.  Afterwards the tokens count as cached (`mgr.commit`).
 
         A batch in which every request brings one token and wants its logits is replayed from a CUDA graph
-        (batch sizes are rounded up to 1, 2, a multiple of 4 up to 32 or a multiple of 8 with stand-in requests that touch only a
+        (batch sizes above 8 are rounded up to a multiple of 4 up to 32 or a multiple of 8 with stand-in requests that touch only a
         spare page; there is a graph per batch size and bucket of context lengths, captured the second time
         the pair is seen); the returned tensor is then a view
         of the graph's own output buffer and holds its values until the next step of the same size."""
@@ -277,19 +292,26 @@ class ModelRunner:
             bucket = self.graph_context_bucket(max(lens))
             skew = self.graph_skew_class(bucket, sum(lens) / len(lens))
         # a graph's block tables are as wide as its bucket of context lengths needs, not as the longest context allowed
-        batch, places = entries, None
-        if skew and len(entries) > 1:
-            # Requests of unequal length are laid out longest first, so that the decode attention starts with its longest blocks and
-            # the short ones fill its last wave; the rows whose logits are wanted keep the order of the
-            # entries.  (Contexts of 130 to 2,300 tokens: 64 requests of the 1B shape 1,660 -> 1,513 us a step, 27 of the 8B
-            # shape 4,677 -> 4,394.)
-            places = sorted(range(len(entries)), key=lambda i: -lens[i])
-            batch = [entries[i] for i in places]
+        # Requests that decode at unequal lengths are laid out longest first (before the prompt portions), so that the decode
+        # attention starts with its longest blocks and the short ones fill its last wave; the rows whose logits are wanted keep
+        # the order of the entries.  (Contexts of 130 to 2,300 tokens: 64 requests of the 1B shape 1,660 -> 1,513 us a step, 27 of
+        # the 8B shape 4,677 -> 4,394, 63 of it beside a portion of 1,985 tokens 31.26 ->
+        # 30.94 ms.)
+        places = self._longest_first(entries, mgr, lens if graph_mode else None, skew)
+        batch = entries if places is None else [entries[i] for i in places]
         hb = self._prepare(batch, mgr, (bucket + self.block_size - 1) // self.block_size if graph_mode else None,
                            self.graph_batch_size(len(entries)) if graph_mode else 0)
         if places is not None:
             rows = hb.pinned.numpy()[hb.seg["rows"][0]:]
-            rows[places] = np.arange(len(places), dtype=np.int32)
+            if graph_mode:
+                rows[places] = np.arange(len(places), dtype=np.int32)
+            else:
+                first = np.zeros(len(entries) + 1, dtype=np.int64)             # where each entry's tokens start
+                for at, i in enumerate(places):
+                    first[at + 1] = first[at] + len(entries[i].tokens)
+                start = {i: int(first[at]) for at, i in enumerate(places)}
+                wanted = [start[i] + int(w) for i, e in enumerate(entries) for w in e.want]
+                rows[:len(wanted)] = wanted
         self.storage.zero_state_slots(mgr.take_fresh_slots())
         key = (hb.S, bucket, skew) if graph_mode else None
         if graph_mode and (key in self._graphs or key in self._seen_sizes):
