@@ -65,6 +65,7 @@ struct Args {
   float* res; long long ldres; const void* norm_w; int norm_w_f32; float* out_sumsq; long long out_ld;
   const bf16* bias;   // [N] or null: added to the sums before anything else is done with them (plain and ROPE forms)
   int plain_act;      // plain form: 0 none, 1 the square of max(sum, 0)
+  int n_blocks;       // groups of rows: more than there are blocks in the launch, if blocks take several in turn
   int planes;         // ROPE: 2 (k and v rows) or 1 (k rows only: a cache whose keys are its values)
 };
 
@@ -102,54 +103,78 @@ __device__ __forceinline__ void issue_rows(uint32_t stage, const bf16* __restric
 // PAIR: the gated form with 8 gate rows and the 8 matching up rows in one group of 16 (rows r and r + 8 belong together):
 // twice the blocks of half the size of a group of gate rows beside a group of up rows, which leaves a shorter tail when
 // the blocks do not fill their last wave.
+//
+// NT 1 (up to 8 rows): a launch has as many blocks as run at a time, and a block takes several groups of rows in turn, its ring
+// of stages running on from one to the next: the next group's weights are on their way while this one's sums meet and leave.
+// A block of its own for every group stopped its part of the stream from its last stage to its successor's first, about a
+// third of a block's life at K = 2,048.  (One request of the 1B shape 711.6 -> 701.4 us a step, five of the 13B shape 8.22 ->
+// 8.14 ms, the life of five requests of the Dizepel design 9.14 -> 8.78 ms; eight of the 8B shape as before, 3.37 ms.)
 template <int NT, int GROUPS, int STAGES, bool ROPE = false, bool PAIR = false>
 __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
   constexpr int kStage = GROUPS * kStageBytes + NT * 8 * kRowBytes;      // W group(s), then x
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g4 = lane >> 2, t4 = lane & 3;
-  const int n0 = blockIdx.x * (PAIR ? 8 : 16);
+  constexpr bool MANY = NT == 1;
+  constexpr int kRing = kWarps * STAGES * kStage, kPartBytes = GROUPS * 16 * 8 * NT * 4;
   const int n_chunks_total = (a.K + kChunkK - 1) / kChunkK;
   // chunk c of warp w is chunk w + 4 c of the row: the four warps walk the same kilobyte of every row together
-  const int c_begin = warp, c_stride = kWarps;
   const int n_chunks = (n_chunks_total - warp + kWarps - 1) / kWarps;
+  const int n_units = MANY ? (a.n_blocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;
+  const int n_total = n_units * n_chunks;
   const uint32_t ring = smem_u32(smem) + warp * (STAGES * kStage);
   const int rows_total = (GROUPS == 2 || PAIR) ? a.up_offset : a.N;       // rows of one group
   // ROPE: rows 0..7 of the block are features f0.., rows 8..15 features f1..: a rotated pair sits 8 rows apart
-  int f0 = n0, f1 = n0 + 8;
-  bool pair8 = false;                                            // the block holds NeoX pairs (i, i + rot/2)
-  if (ROPE && a.inv_freq && a.is_neox) {
-    const int head = n0 / a.head_dim, j = (n0 % a.head_dim) / 16;
-    if (head < a.n_q_heads + a.n_kv_heads && j * 16 < a.rot_dim) {
-      f0 = head * a.head_dim + 8 * j;
-      f1 = f0 + a.rot_dim / 2;
-      pair8 = true;
+  struct Rows { int n0, f0, f1; bool pair8; };                   // pair8: the group holds NeoX pairs (i, i + rot/2)
+  auto rows_of = [&](int blk) -> Rows {
+    Rows r;
+    r.n0 = blk * (PAIR ? 8 : 16);
+    r.f0 = r.n0; r.f1 = r.n0 + 8; r.pair8 = false;
+    if (ROPE && a.inv_freq && a.is_neox) {
+      const int head = r.n0 / a.head_dim, j = (r.n0 % a.head_dim) / 16;
+      if (head < a.n_q_heads + a.n_kv_heads && j * 16 < a.rot_dim) {
+        r.f0 = head * a.head_dim + 8 * j;
+        r.f1 = r.f0 + a.rot_dim / 2;
+        r.pair8 = true;
+      }
     }
-  }
-  const int hi_off = f1 - f0 - 8;
+    return r;
+  };
 
-  auto issue_w = [&](int c) {
-    const uint32_t st = ring + (c % STAGES) * kStage;
-    const int k0 = (c_begin + c * c_stride) * kChunkK;
-    if (ROPE) issue_rows<16>(st, a.w + (size_t)f0 * a.ldw, a.ldw, 16, k0, a.K, lane, hi_off);
+  // the stage that is asked for next: its group of rows, its chunk of them, its place in the ring (x follows the chunk alone)
+  int w_blk = blockIdx.x, w_chunk = 0, w_slot = 0, x_chunk = 0, x_slot = 0;
+  Rows w_rows = rows_of(w_blk);
+  auto issue_w = [&]() {
+    const uint32_t st = ring + w_slot * kStage;
+    const int k0 = (warp + w_chunk * kWarps) * kChunkK, n0 = w_rows.n0;
+    if (ROPE) issue_rows<16>(st, a.w + (size_t)w_rows.f0 * a.ldw, a.ldw, 16, k0, a.K, lane, w_rows.f1 - w_rows.f0 - 8);
     else if (PAIR) issue_rows<16>(st, a.w + (size_t)n0 * a.ldw, a.ldw, min(8, rows_total - n0), k0, a.K, lane, a.up_offset - 8, true);
     else issue_rows<16>(st, a.w + (size_t)n0 * a.ldw, a.ldw, rows_total - n0, k0, a.K, lane);
     if (GROUPS == 2)
       issue_rows<16>(st + kStageBytes, a.w + (size_t)(a.up_offset + n0) * a.ldw, a.ldw, rows_total - n0, k0, a.K, lane);
+    if (++w_slot == STAGES) w_slot = 0;
+    if (++w_chunk == n_chunks) {
+      w_chunk = 0;
+      if (MANY) {
+        w_blk += gridDim.x;
+        w_rows = rows_of(w_blk);
+      }
+    }
   };
-  auto issue_x = [&](int c) {
-    const uint32_t st = ring + (c % STAGES) * kStage;
-    issue_rows<8 * NT>(st + GROUPS * kStageBytes, a.x, a.ldx, a.M, (c_begin + c * c_stride) * kChunkK, a.K, lane);
+  auto issue_x = [&]() {
+    const uint32_t st = ring + x_slot * kStage;
+    issue_rows<8 * NT>(st + GROUPS * kStageBytes, a.x, a.ldx, a.M, (warp + x_chunk * kWarps) * kChunkK, a.K, lane);
+    if (++x_slot == STAGES) x_slot = 0;
+    if (++x_chunk == n_chunks) x_chunk = 0;
   };
-  auto issue = [&](int c) { issue_w(c); issue_x(c); };
   // The weights do not depend on the kernel before this one: their first stages are requested while that
   // kernel may still be running; x is read only after it has finished.
   pdl_launch_dependents();
   for (int s = 0; s < STAGES - 1; ++s)
-    if (s < n_chunks) issue_w(s);
+    if (s < n_total) issue_w();
   pdl_wait();
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < n_chunks) issue_x(s);
+    if (s < n_total) issue_x();
     cp_async_commit();
   }
 
@@ -175,6 +200,11 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
     }
   };
   if (a.in_sumsq) load_ss(0);
+  int asked = STAGES - 1, slot = 0;                              // stages asked for so far; the place of the next one to use
+  for (int unit = 0; unit < n_units; ++unit) {
+  const Rows rows = rows_of(blockIdx.x + unit * gridDim.x);
+  const int n0 = rows.n0, f0 = rows.f0, f1 = rows.f1;
+  const bool pair8 = rows.pair8;
   // residual form: the residual values and norm weights of this thread's results, asked for before the loop
   float e_res[NT], e_nw[NT];
   if (!ROPE && !PAIR && GROUPS == 1 && a.res) {
@@ -213,9 +243,11 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
   for (int c = 0; c < n_chunks; ++c) {
     cp_async_wait<STAGES - 2>();
     __syncwarp();
-    if (c + STAGES - 1 < n_chunks) issue(c + STAGES - 1);
+    if (asked < n_total) { issue_w(); issue_x(); }
+    ++asked;
     cp_async_commit();
-    const uint32_t st = ring + (c % STAGES) * kStage;
+    const uint32_t st = ring + slot * kStage;
+    if (++slot == STAGES) slot = 0;
     const uint32_t xs = st + GROUPS * kStageBytes;
     const int mi = lane >> 3, r = lane & 7;
 #pragma unroll
@@ -249,11 +281,14 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
       }
     }
   }
-  cp_async_wait<0>();
-  __syncwarp();
-
-  // partial sums of the four warps: [warp][group][row 16][token 8 NT], added in warp order
-  float* part = reinterpret_cast<float*>(smem + warp * (STAGES * kStage));
+  // partial sums of the four warps: [warp][group][row 16][token 8 NT], added in warp order; behind the rings, or where a
+  // warp's ring was
+  if (!MANY) {
+    cp_async_wait<0>();
+    __syncwarp();
+  }
+  auto part_of = [&](int w) { return reinterpret_cast<float*>(MANY ? smem + kRing + w * kPartBytes : smem + w * (STAGES * kStage)); };
+  float* part = part_of(warp);
 #pragma unroll
   for (int g = 0; g < GROUPS; ++g)
 #pragma unroll
@@ -264,9 +299,10 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
       base[(g4 + 8) * (8 * NT) + t * 8 + t4 * 2] = acc[g][t][2];
       base[(g4 + 8) * (8 * NT) + t * 8 + t4 * 2 + 1] = acc[g][t][3];
     }
-  // prenormed input: token m's factor, kept in the region of the warp that summed it
+  // prenormed input: token m's factor, kept behind the partial sums, or in the region of the warp that summed it
   constexpr int kFactorOff = 2048;                                 // behind the largest set of partial sums
-  if (a.in_sumsq) {
+  auto factor_of = [&](int w) { return reinterpret_cast<float*>(MANY ? smem + kRing + kWarps * kPartBytes : smem + w * (STAGES * kStage) + kFactorOff); };
+  if (a.in_sumsq && unit == 0) {
     float row_ss = 0.f;
     for (int q0 = 0;;) {
 #pragma unroll
@@ -278,13 +314,13 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
 #pragma unroll
     for (int o = kTPR / 2; o > 0; o >>= 1) row_ss += __shfl_xor_sync(0xffffffffu, row_ss, o);
     if (threadIdx.x % kTPR == 0 && threadIdx.x / kTPR < a.M)
-      reinterpret_cast<float*>(smem + warp * (STAGES * kStage) + kFactorOff)[threadIdx.x / kTPR] =
+      factor_of(warp)[threadIdx.x / kTPR] =
           1.0f / sqrtf(row_ss / (float)a.in_width + a.in_eps);
   }
   __syncthreads();
   auto factor = [&](int m) -> float {
     if (!a.in_sumsq || m >= a.M) return 1.0f;
-    return reinterpret_cast<const float*>(smem + ((m * kTPR) >> 5) * (STAGES * kStage) + kFactorOff)[m];
+    return factor_of((m * kTPR) >> 5)[m];
   };
   if constexpr (ROPE) {
     // one (token, feature) per thread and pass; the partner of a rotated pair is 8 lanes away (NeoX) or the neighbour
@@ -296,7 +332,7 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
       float sum = 0.f;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w)
-        sum += reinterpret_cast<const float*>(smem + w * (STAGES * kStage))[row * (8 * NT) + m];
+        sum += part_of(w)[row * (8 * NT) + m];
       sum *= factor(m);
       const int n = row < 8 ? f0 + row : f1 + row - 8;                  // feature among q, k, v (and the rows behind them)
       if (a.bias) sum += __bfloat162float(a.bias[n]);
@@ -337,7 +373,7 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
       float sum = 0.f;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w)
-        sum += reinterpret_cast<const float*>(smem + w * (STAGES * kStage))[row * (8 * NT) + m];
+        sum += part_of(w)[row * (8 * NT) + m];
       sum *= factor(m);
       const float up = __shfl_down_sync(0xffffffffu, sum, 8);
       if (row >= 8 || m >= a.M || n0 + row >= rows_total) continue;
@@ -358,7 +394,7 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
         float s = 0.f;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w)
-          s += reinterpret_cast<const float*>(smem + w * (STAGES * kStage))[g * (16 * 8 * NT) + row * (8 * NT) + m];
+          s += part_of(w)[g * (16 * 8 * NT) + row * (8 * NT) + m];
         v[g] = s * f;
       }
       float r = GROUPS == 2 ? act_apply(v[0], a.act) * v[GROUPS - 1] : v[0];
@@ -376,25 +412,42 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
         float sq = nr * nr;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (row == 0 && m < a.M) a.out_sumsq[(size_t)m * a.out_ld + blockIdx.x] = sq;
+        if (row == 0 && m < a.M) a.out_sumsq[(size_t)m * a.out_ld + n0 / 16] = sq;
       } else if (ok) {
         if (a.out_f32) reinterpret_cast<float*>(a.out)[(size_t)m * a.ldo + n0 + row] = r;
         else reinterpret_cast<bf16*>(a.out)[(size_t)m * a.ldo + n0 + row] = __float2bfloat16_rn(r);
       }
     }
   }
+  if (unit + 1 < n_units) __syncthreads();                       // the sums have been read before the next group's are written
+  }
+  if (MANY) cp_async_wait<0>();
+}
+
+static int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
+  }
+  return n;
 }
 
 template <int NT, int GROUPS, int STAGES, bool ROPE = false, bool PAIR = false>
 static int launch(const Args& a, int rows, cudaStream_t s) {
-  const int smem = kWarps * STAGES * (GROUPS * kStageBytes + NT * 8 * kRowBytes);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(skinny_kernel<NT, GROUPS, STAGES, ROPE, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto* kernel = skinny_kernel<NT, GROUPS, STAGES, ROPE, PAIR>;
+  constexpr int smem = kWarps * STAGES * (GROUPS * kStageBytes + NT * 8 * kRowBytes) + (NT == 1 ? kWarps * GROUPS * 16 * 8 * 4 + 32 : 0);
+  static int slots = 0;                                          // blocks that run at a time
+  if (slots == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarps * 32, smem);
     if (e != cudaSuccess) return (int)e;
-    configured = true;
+    slots = (per_sm > 0 ? per_sm : 1) * sm_count();
   }
-  return launch_pdl(skinny_kernel<NT, GROUPS, STAGES, ROPE, PAIR>, dim3(ceil_div(rows, PAIR ? 8 : 16)), dim3(kWarps * 32), smem, s, a);
+  Args b = a;
+  b.n_blocks = ceil_div(rows, PAIR ? 8 : 16);
+  return launch_pdl(kernel, dim3(NT == 1 && b.n_blocks > slots ? slots : b.n_blocks), dim3(kWarps * 32), smem, s, b);
 }
 
 #ifndef LMSF_SKINNY_STAGES
@@ -431,15 +484,6 @@ constexpr int kStagesFused = LMSF_SKINNY_STAGES_FUSED;
 #endif
 constexpr int kStagesFew = LMSF_SKINNY_STAGES_FEW, kStagesOne = LMSF_SKINNY_STAGES_ONE;
 constexpr int kStagesFew16 = LMSF_SKINNY_STAGES_FEW_M16, kStagesOne16 = LMSF_SKINNY_STAGES_ONE_M16;
-
-static int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
-  }
-  return n;
-}
 
 // The plain, residual, prenormed and q/k/v forms (one group of 16 rows a block): the ring's depth by the number of blocks.
 template <bool ROPE>
