@@ -240,17 +240,14 @@ class ModelRunner:
 
     @staticmethod
     def graph_reach(bucket: int, max_ctx: int) -> int:
-        """The context length that a graph's splits are planned for: in the first bucket 256, 512 or the bucket, in a later one
-        three quarters of it or the bucket, whichever the longest context fits.  (Planned for 1,024 keys, short contexts got
-        splits without keys: the attention of 63 requests of 16 to 300 keys took 31.1 us with 2 splits and takes 13.4 with one, of
-        the 1B shape 21.7 with 4 and 8.1 with one, of one request of 97 keys 4.3 and 2.8.  Planned for 1,536 keys, 8 requests
-        of the 8B shape at 2,047 got 3 splits and 18.9 us, where 4 take 16.4: REACH_FIGURES.)"""
-        if bucket > 1024:
-            return bucket - bucket // 4 if max_ctx <= bucket - bucket // 4 else bucket
+        """The context length that a graph's splits are planned for: its bucket, or in the first bucket 256 or 512 where the
+        longest context is no longer.  (Planned for 1,024 keys, short contexts got splits without keys: the attention of 63
+        requests of 16 to 300 keys took 31.1 us with 2 splits and takes 13.4 with one, of the 1B shape 21.7 with 4 and 8.1 with
+        one, of one request of 97 keys 4.3 and 2.8.)"""
         r = 256
         while r < max_ctx:
             r *= 2
-        return min(r, bucket)
+        return min(r, bucket) if bucket <= 1024 else bucket
 
     @staticmethod
     def graph_skew_class(bucket: int, mean_ctx: float) -> int:
@@ -349,10 +346,10 @@ class ModelRunner:
         if g is None:
             static_in = self._upload(hb)
             ctx, rows = self._context(hb, static_in)
-            # launch geometry must not depend on the step, only on its graph: the decode attention plans its splits for the
-            # longest contexts that the graph serves
+            # launch geometry must not depend on the step, only on its bucket: the decode attention plans its splits
+            # for the middle of the bucket's context lengths (the bucket below ends at half its top)
             reach = key[3]
-            ctx.extras["decode_max_ctx"] = reach
+            ctx.extras["decode_max_ctx"] = reach - reach // 4 if reach > 1024 else reach
             # the middle of the graph's class of means: between reach / (2 << c) and twice that (the last class: and
             # below); class 0 plans as if all contexts were as long as the longest
             ctx.extras["decode_mean_ctx"] = reach * 3 / (4 << key[2]) if key[2] else ctx.extras["decode_max_ctx"]

@@ -66,6 +66,23 @@ def test_buckets_of_context_lengths():
     assert b(1) == 300 and b(300) == 300
 
 
+def test_what_a_decode_graph_is_planned_for():
+    """Above 1,024 keys one plan serves the whole bucket: it changes with the bucket, not within it."""
+    from lmsf_b200.engine.model_runner import ModelRunner
+    r = ModelRunner.graph_reach
+    assert [r(1024, n) for n in (1, 256, 257, 512, 513, 1024)] == [256, 256, 512, 512, 1024, 1024]
+    assert [r(300, n) for n in (1, 256, 257, 300)] == [256, 256, 300, 300] and r(100, 100) == 100
+    for bucket in (2048, 4096, 8192, 10000):
+        assert {r(bucket, n) for n in range(bucket // 2 + 1, bucket + 1, 97)} == {bucket}
+
+
+def test_sizes_of_decode_graphs():
+    from lmsf_b200.engine.model_runner import ModelRunner
+    size = ModelRunner.graph_batch_size
+    assert [size(n) for n in range(1, 9)] == list(range(1, 9))
+    assert [size(n) for n in (9, 12, 13, 27, 32, 33, 40, 41, 64, 255)] == [12, 12, 16, 28, 32, 40, 40, 48, 64, 256]
+
+
 def test_token_history_counts_like_a_recount():
     rng = random.Random(0)
     for _ in range(20):
