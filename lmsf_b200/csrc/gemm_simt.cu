@@ -100,6 +100,7 @@ struct F32Args {
   float* C; const float* A; const float* W;
   int M, N, K;
   long long lda, ldw, ldc, batch_a, batch_w, batch_c;
+  int w_constant;        // no kernel of the step writes W: it may be read before the kernel ahead has ended
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -120,8 +121,9 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // Up to 16 rows of A: a stream over W.  A block takes 16 rows of W, its warp w the parts 2 w (lanes 0..15, a row of W
 // each) and 2 w + 1 (lanes 16..31), through a ring of its own of cp.async stages of 32 k: 4 KB of W (chunks of 16 bytes
 // swizzled by the row, so that eight lanes read eight different banks) and the matching x, which all lanes of a part read
-// together.  Bound by the stream: with five stages (three at 16 rows) two blocks fit an SM and keep 128 KB of W asked for.  W's first stages
-// are asked for before the kernel before this one has ended.  One launch after the
+// together.  Bound by the stream: with five stages (three at 16 rows) two blocks fit an SM and keep 128 KB of W asked for.  Where the caller
+// says that W is a weight, its first stages are asked for before the kernel before this one has ended, and the kernel after this one
+// may start as early.  Any other W may be what that kernel writes: then everything waits, as in plain stream order.  One launch after the
 // other on different weights at 3 rows: 128,256 x 2,048 in 151 us (7.0 TB/s), 16,384 x 2,048 in 25 us (5.3), 2,048 x 8,192 in
 // 14 us (4.8); 31 and 25 us for the last two with single FMAs and an address per copy.  (Prompts of 515 tokens and 12 decoded
 // tokens for three requests, Llama-3.2-1B: 294 -> 50.8 ms with this kernel and the next.)
@@ -172,12 +174,17 @@ __global__ void __launch_bounds__(128) f32_few_rows_kernel(F32Args a) {
       cp16(st + row * 128 + (ch << 4), ok ? A + (size_t)m * a.lda + k : A, ok);
     }
   };
-  pdl_launch_dependents();
-  for (int s = 0; s < kFewStages - 1; ++s)
-    if (s < n_st) issue_w(s);
+  if (a.w_constant) {
+    pdl_launch_dependents();
+    for (int s = 0; s < kFewStages - 1; ++s)
+      if (s < n_st) issue_w(s);
+  }
   pdl_wait();
   for (int s = 0; s < kFewStages - 1; ++s) {
-    if (s < n_st) issue_x(s);
+    if (s < n_st) {
+      if (!a.w_constant) issue_w(s);
+      issue_x(s);
+    }
     cp_commit();
   }
 
@@ -435,10 +442,11 @@ static int launch_f32(const F32Args& a, int batch, cudaStream_t s) {
 
 // `batch` products in one launch: product b reads A + b * batch_a and W + b * batch_w and writes C + b * batch_c
 // (elements).  The heads of one activation matrix are such a batch: batch_a = head size, lda = the row stride.
-// in_dtype: type of A and W; out_dtype: type of C.  Leading dimensions in elements.
+// in_dtype: type of A and W; out_dtype: type of C.  Leading dimensions in elements.  w_constant: W is a weight, which no kernel
+// of the step writes; 0: W may have been written by the launch just before this one.
 LMSF_API int lmsf_gemm_tn_simt_batched(void* C, const void* A, const void* W, int M, int N, int K, long long lda,
                                        long long ldw, long long ldc, int batch, long long batch_a, long long batch_w,
-                                       long long batch_c, int in_dtype, int out_dtype, void* stream) {
+                                       long long batch_c, int in_dtype, int out_dtype, int w_constant, void* stream) {
   using namespace lmsf;
   if (M <= 0 || N <= 0 || batch <= 0) return 0;
   if (K <= 0) LMSF_REFUSE("gemm: K=%d must be positive", K);
@@ -450,7 +458,8 @@ LMSF_API int lmsf_gemm_tn_simt_batched(void* C, const void* A, const void* W, in
   const bool wide = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && batch_a % 4 == 0 && batch_w % 4 == 0 &&
                     (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
   if (in_dtype == LMSF_F32 && out_dtype == LMSF_F32 && wide && ceil_div(N, TN) <= 65535)
-    return launch_f32(F32Args{(float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c}, batch, s);
+    return launch_f32(F32Args{(float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c,
+                              w_constant ? 1 : 0}, batch, s);
   if (in_dtype == LMSF_F32 && out_dtype == LMSF_F32)
     gemm_tn_kernel<float, float><<<grid, 256, 0, s>>>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);
   else if (in_dtype == LMSF_BF16 && out_dtype == LMSF_BF16)
@@ -463,6 +472,6 @@ LMSF_API int lmsf_gemm_tn_simt_batched(void* C, const void* A, const void* W, in
 }
 
 LMSF_API int lmsf_gemm_tn_simt(void* C, const void* A, const void* W, int M, int N, int K, long long lda,
-                               long long ldw, long long ldc, int in_dtype, int out_dtype, void* stream) {
-  return lmsf_gemm_tn_simt_batched(C, A, W, M, N, K, lda, ldw, ldc, 1, 0, 0, 0, in_dtype, out_dtype, stream);
+                               long long ldw, long long ldc, int in_dtype, int out_dtype, int w_constant, void* stream) {
+  return lmsf_gemm_tn_simt_batched(C, A, W, M, N, K, lda, ldw, ldc, 1, 0, 0, 0, in_dtype, out_dtype, w_constant, stream);
 }

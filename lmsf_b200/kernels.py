@@ -423,9 +423,10 @@ def bias_add(x: torch.Tensor, bias: torch.Tensor):
 
 # ----------------------------------------------------------------------------- SIMT matrix product
 
-def gemm_tn_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
+def gemm_tn_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, w_constant: bool = False):
     """out[M, N] = a[M, K] w[N, K]^T, float32 FMA accumulation in a fixed order, whatever M is (true 32-bit when
-    a, w are float32: sixteen sums over ascending k, added up)."""
+    a, w are float32: sixteen sums over ascending k, added up).  w_constant: w is a weight that no kernel of the step writes; a
+    product of few rows then reads it while the kernel before it is still running."""
     M, K = a.shape
     N = w.shape[0]
     if w.shape[1] != K or out.shape != (M, N) or a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
@@ -433,10 +434,10 @@ def gemm_tn_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
     if a.dtype != w.dtype:
         raise KernelError("gemm: a and w must share one dtype")
     f = _func("gemm_simt.cu", "lmsf_gemm_tn_simt",
-              [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int,
+              [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int, c_int,
                c_void_p])
     rc = f(_ptr(out), _ptr(a), _ptr(w), M, N, K, a.stride(0), w.stride(0), out.stride(0), dtype_code(a.dtype),
-           dtype_code(out.dtype), _stream())
+           dtype_code(out.dtype), int(w_constant), _stream())
     _check(rc, "gemm_simt.cu", "lmsf_gemm_simt")
 
 
@@ -1460,9 +1461,10 @@ def attention_shared_kv(out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor,
     _check(rc, "attention_generic.cu", "lmsf_attention_generic")
 
 
-def gemm_tn_simt_batched(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
+def gemm_tn_simt_batched(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, w_constant: bool = False):
     """out[:, b, :] = a[:, b, :] w[b]^T for every b.  a: [M, B, K], out: [M, B, N] (views: the last dimension
-    contiguous, any row and batch strides); w: [B, N, K].  float32 FMA accumulation in the order of `gemm_tn_simt`."""
+    contiguous, any row and batch strides); w: [B, N, K].  float32 FMA accumulation in the order of `gemm_tn_simt`;
+    w_constant as there."""
     M, B, K = a.shape
     N = w.shape[1]
     if w.shape != (B, N, K) or out.shape != (M, B, N) or a.stride(2) != 1 or w.stride(2) != 1 or out.stride(2) != 1 \
@@ -1470,9 +1472,9 @@ def gemm_tn_simt_batched(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor):
         raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)}")
     f = _func("gemm_simt.cu", "lmsf_gemm_tn_simt_batched",
               [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_longlong,
-               c_longlong, c_longlong, c_int, c_int, c_void_p])
+               c_longlong, c_longlong, c_int, c_int, c_int, c_void_p])
     rc = f(_ptr(out), _ptr(a), _ptr(w), M, N, K, a.stride(0), w.stride(1), out.stride(0), B, a.stride(1), w.stride(0),
-           out.stride(1), dtype_code(a.dtype), dtype_code(out.dtype), _stream())
+           out.stride(1), dtype_code(a.dtype), dtype_code(out.dtype), int(w_constant), _stream())
     _check(rc, "gemm_simt.cu", "lmsf_gemm_simt")
 
 

@@ -33,7 +33,8 @@ def _skinny_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def matmul_tn(x: Union[torch.Tensor, Prenormed], w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
               bias: Optional[torch.Tensor] = None, act: Optional[str] = None) -> torch.Tensor:
-    """x [M, K] times w [N, K] transposed -> [M, N] in `out_dtype` (default: x's dtype), plus `bias` [N] if given.  The
+    """x [M, K] times w [N, K], a weight, transposed -> [M, N] in `out_dtype` (default: x's dtype), plus `bias` [N] if given.  (The
+    kernels for few rows read w while the step's kernel before them still runs: no kernel of the step may write it.)  The
     bfloat16 products add a bfloat16 bias to their float32 sums before they round (the reference adds it afterwards, in a
     step of its own: layers/linear.rs:100-104); otherwise a kernel adds it after the product.  `act` "relu2": the square of
     max(result, 0).  x may be a `Prenormed`: the weight-streaming kernel divides its sums by the rows' root mean square."""
@@ -71,7 +72,7 @@ def _product_tn(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32:
         out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
-        kernels.gemm_tn_simt(out, x, w)
+        kernels.gemm_tn_simt(out, x, w, w_constant=True)
         return out if out_dtype == torch.float32 else out.to(out_dtype)
     if _skinny_takes(x, w) and out_dtype in (torch.bfloat16, torch.float32):
         out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
@@ -89,19 +90,20 @@ def _product_tn(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
                 raise
             _MM_HAS_OUT_DTYPE = False
     out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
-    kernels.gemm_tn_simt(out, x, w)
+    kernels.gemm_tn_simt(out, x, w, w_constant=True)
     return out
 
 
 def batched_matmul_tn(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """out[:, b, :] = a[:, b, :] w[b]^T for every b: one product per head of an activation matrix.
-    a: [M, B, K] and out: [M, B, N] are views with a contiguous last dimension; w: [B, N, K].
+    a: [M, B, K] and out: [M, B, N] are views with a contiguous last dimension; w: [B, N, K], weights (read ahead as in
+    `matmul_tn`).
     bfloat16 with more than 16 rows: the library's batched product; else this package's FFMA kernel (true 32-bit
     for float32; few rows in bfloat16, where the product is a stream over w)."""
     if a.dtype == torch.bfloat16 and a.shape[0] > kernels.SKINNY_MAX_M:
         torch.bmm(a.transpose(0, 1), w.transpose(1, 2), out=out.transpose(0, 1))
     else:
-        kernels.gemm_tn_simt_batched(out, a, w)
+        kernels.gemm_tn_simt_batched(out, a, w, w_constant=True)
     return out
 
 

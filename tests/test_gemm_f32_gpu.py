@@ -45,3 +45,39 @@ def test_batches_of_products(M, N, K):
     kernels.gemm_tn_simt_batched(out, a, w)
     for b in range(5):
         assert torch.equal(out[:, b], _product(a[:, b].contiguous(), w[b]))
+
+
+@pytest.mark.parametrize("M", [1, 3, 16])
+def test_a_second_operand_that_the_launch_before_has_written(M):
+    """Only what the caller calls a weight is read ahead of the launch before: a product whose w is the output of a product that lets
+    its successor start early gives the bits that it gives when everything before it has ended."""
+    from lmsf_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rows, K, N = 16, 4096, 8192                              # the first product takes tens of microseconds
+    x, weight = torch.randn(rows, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    a = torch.randn(M, N, device="cuda", generator=g)
+    w = torch.empty(rows, N, device="cuda")
+    out, want = torch.empty(M, rows, device="cuda"), torch.empty(M, rows, device="cuda")
+    w3, a3 = w.view(4, 4, N), a.view(M, 4, N // 4)           # as a batch: w[b] = rows 4 b .. of w, its first N / 4 values
+    out3, want3 = torch.empty(M, 4, 4, device="cuda"), torch.empty(M, 4, 4, device="cuda")
+
+    def first():
+        w.fill_(float("nan"))
+        torch.cuda.synchronize()
+        kernels.gemm_tn_simt(w, x, weight, w_constant=True)
+
+    first()
+    torch.cuda.synchronize()
+    kernels.gemm_tn_simt(want, a, w)
+    kernels.gemm_tn_simt_batched(want3, a3, w3[:, :, :N // 4])
+    assert bool(torch.isfinite(want).all()) and bool(torch.isfinite(want3).all())
+    for _ in range(5):
+        first()
+        kernels.gemm_tn_simt(out, a, w)
+        assert torch.equal(out, want)
+        first()
+        kernels.gemm_tn_simt_batched(out3, a3, w3[:, :, :N // 4])
+        assert torch.equal(out3, want3)
+    # the second one as what it is, after a synchronisation: the same bits
+    kernels.gemm_tn_simt(out, a, w, w_constant=True)
+    assert torch.equal(out, want)
