@@ -221,7 +221,6 @@ __global__ void __launch_bounds__(kWarps * 32) attention_staged_kernel(GenericAt
   int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
   if (a.chunk > 0) lo = max(lo, pos - pos % a.chunk);
   const int keep = lo > 0 ? min(a.keep_first, lo) : 0;
-  const float hb = a.head_bias ? a.head_bias[head] : 0.f;
   const int* table = a.block_table + (size_t)a.token_seq[t] * a.max_blocks;
   const size_t head_off = (size_t)kvh * a.block_size * hd;
   const size_t v_off = a.shared_kv ? 0 : (size_t)a.n_kv_heads * a.block_size * hd;
@@ -253,7 +252,8 @@ __global__ void __launch_bounds__(kWarps * 32) attention_staged_kernel(GenericAt
 
   int tile = from(warp);
   long long row = tile * 32 <= pos ? row_of(tile) : -1;
-  pdl_wait();
+  pdl_wait();                                              // so far the step's tables alone were read, which no kernel of a step writes
+  const float hb = a.head_bias ? a.head_bias[head] : 0.f;
   if (tile * 32 <= pos) {
     fetch(ks_addr, row, 0);
     fetch(vs_addr, row, v_off);
@@ -287,11 +287,13 @@ __global__ void __launch_bounds__(kWarps * 32) attention_staged_kernel(GenericAt
     if (more) fetch(ks_addr, next_row, 0);
     else cp_commit();
     float p = 0.f;
+    bool some = true;                                      // the tile has a weight (uniform over the warp)
     if (a.sigmoid) {   // every key on its own: no running maximum, no denominator
       if (row >= 0) p = 1.0f / (1.0f + expf(-s));
     } else {
       const float m_new = fmaxf(m, warp_max(s));
-      if (m_new != -INFINITY) {   // something has been seen (uniform over the warp)
+      some = m_new != -INFINITY;   // something has been seen
+      if (some) {
         if (row >= 0) p = expf(s - m_new);
         const float alpha = expf(m - m_new);
         l = l * alpha + warp_sum(p);
@@ -302,11 +304,13 @@ __global__ void __launch_bounds__(kWarps * 32) attention_staged_kernel(GenericAt
     }
     cp_wait<1>();
     __syncwarp();
+    if (some) {                    // values behind scores that are all minus infinity are left alone
 #pragma unroll 8
-    for (int j = 0; j < 32; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      if (lane < hd) acc[0] = fmaf(pj, vs[j * stride + lane], acc[0]);
-      if (lane + 32 < hd) acc[1] = fmaf(pj, vs[j * stride + lane + 32], acc[1]);
+      for (int j = 0; j < 32; ++j) {
+        const float pj = __shfl_sync(0xffffffffu, p, j);
+        if (lane < hd) acc[0] = fmaf(pj, vs[j * stride + lane], acc[0]);
+        if (lane + 32 < hd) acc[1] = fmaf(pj, vs[j * stride + lane + 32], acc[1]);
+      }
     }
     __syncwarp();
     if (more) fetch(vs_addr, next_row, v_off);
