@@ -7,6 +7,7 @@ only the tokens it is given and returns float32 logits at the wanted places; sam
 """
 from __future__ import annotations
 
+from collections import OrderedDict
 from dataclasses import dataclass, field
 from typing import Hashable, List, Optional, Sequence, Tuple
 
@@ -90,7 +91,11 @@ class ModelRunner:
         self.enforce_eager = enforce_eager
         self.max_graph_batch = max_num_seqs
         self.graph_safe = all(getattr(part, "graph_safe", False) for part, _ in model.parts_with_specs())
-        self._graphs = {}
+        self._graphs = OrderedDict()                               # least recently used first
+        # Every graph keeps its logits alive.  Together they may hold a 64th of the device's memory (2.8 GB: 86 graphs of 64 requests
+        # and 128,256 logits) and half of what lies free beside the cache and a step's own buffers; then the one unused for longest goes.
+        free, total = torch.cuda.mem_get_info(device)
+        self.graph_output_bytes = max(0, min(total // 64, (free - activation_reserve_bytes) // 2))
         self._seen_sizes = set()
         self._graph_pool = None
         self._capture_stream = None
@@ -372,6 +377,8 @@ class ModelRunner:
             n_launches = kernels.launch_count() - before
             kernels.add_launches(-n_launches)                      # recorded, not run
             g = self._graphs[key] = (graph, static_in, static_out, n_launches, hb.total)
+            self._drop_old_graphs()
+        self._graphs.move_to_end(key)
         graph, static_in, static_out, n_launches, total = g
         if total != hb.total:
             raise StepError("the layout of a replayed batch changed")
@@ -380,6 +387,18 @@ class ModelRunner:
         graph.replay()
         kernels.add_launches(n_launches)
         return static_out
+
+    def _drop_old_graphs(self) -> None:
+        """Gives back the graphs used least recently until the outputs of the others fit (the newest always stays).  Logits that a
+        caller still holds stay as they are."""
+        held = sum(g[2].numel() * g[2].element_size() for g in self._graphs.values())
+        if held <= self.graph_output_bytes or len(self._graphs) < 2:
+            return
+        torch.cuda.synchronize(self.device)                        # none of them is still running
+        while held > self.graph_output_bytes and len(self._graphs) > 1:
+            _, (graph, _, out, _, _) = self._graphs.popitem(last=False)
+            graph.reset()
+            held -= out.numel() * out.element_size()
 
     def decode_step(self, entries: Sequence[StepEntry], mgr: CacheManager) -> torch.Tensor:
         """A step whose entries all bring one token; device errors are left for the caller to check."""

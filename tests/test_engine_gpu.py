@@ -397,3 +397,44 @@ def test_a_windowed_prompt_longer_than_the_cache_runs_in_portions():
         assert o.outputs[0].token_ids == ref
     llm.engine.cache.check_invariants()
     assert llm.engine.cache.num_free_pages() == 4
+
+
+def test_decode_graphs_are_bounded_by_what_their_outputs_hold():
+    """Every graph keeps its logits alive; the ones used least recently go when they hold too much together.  Steps give the same
+    bits with any bound, and logits of a graph that has gone stay what they were."""
+    from lmsf_b200.engine.factory import build_model
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    cfg = util.CONFIGS["A"]
+    model, _, tdt = build_model(util.model_folder("A", "bfloat16", 0.15), "bfloat16", "cuda:0")
+    sizes = [3, 3, 3, 1, 1, 1, 6, 6, 6, 12, 12, 3, 3, 2, 2, 6, 1, 4, 4, 9, 9, 3]
+    row = cfg["vocab_size"] * 4
+
+    def run(bound):
+        runner = ModelRunner(model, tdt, torch.device("cuda:0"), 8, num_blocks=128, max_num_seqs=12)
+        assert runner.graph_output_bytes > 0
+        if bound is not None:
+            runner.graph_output_bytes = bound
+        mgr = runner.make_cache_manager()
+        for i in range(12):
+            mgr.add(i)
+        runner.step([StepEntry(i, util.random_ids(40 + i % 3, cfg["vocab_size"], i), []) for i in range(12)], mgr)
+        out, kept = [], None
+        for k, n in enumerate(sizes):
+            lg = runner.step([StepEntry(i, [(7 * k + i) % cfg["vocab_size"]], [0]) for i in range(n)], mgr)
+            if k == 2:
+                kept = lg                                     # replayed: a view of the graph's own buffer
+            out.append(lg.clone())
+            if k == 10:
+                assert torch.equal(kept, out[2])              # until the next step of three requests
+            if bound is not None:
+                rows = [key[0] for key in runner._graphs]
+                assert sum(rows) * row <= bound or len(rows) == 1
+        assert len(runner._graphs) > 0
+        return out, len(runner._graphs)
+
+    free, n_free = run(None)
+    assert n_free == 6                                        # 1, 2, 3, 4, 6 and 12 requests
+    for bound in (0, 9 * row, 20 * row):
+        got, n = run(bound)
+        assert 1 <= n < n_free
+        assert all(torch.equal(a, b) for a, b in zip(free, got))
