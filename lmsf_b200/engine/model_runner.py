@@ -282,6 +282,15 @@ class ModelRunner:
             return None
         return sorted(range(len(entries)), key=lambda i: -lens[i])
 
+    @staticmethod
+    def _wanted_rows(entries: Sequence[StepEntry], places: Sequence[int]) -> List[int]:
+        """Where the wanted tokens lie in a batch laid out in the order `places`: in the order of the entries and of their `want`."""
+        start, at = [0] * len(entries), 0
+        for i in places:
+            start[i] = at
+            at += len(entries[i].tokens)
+        return [start[i] + int(w) for i, e in enumerate(entries) for w in e.want]
+
     def _patch(self, hb: "_HostBatch", dev: torch.Tensor, pending_tokens: Optional[torch.Tensor]) -> None:
         if not hb.has_patches:
             return
@@ -298,8 +307,8 @@ class ModelRunner:
 
         A batch in which every request brings one token and wants its logits is replayed from a CUDA graph
         (batch sizes above 8 are rounded up to a multiple of 4 up to 32 or a multiple of 8 with stand-in requests that touch only a
-        spare page; there is a graph per batch size and bucket of context lengths, captured the second time
-        the pair is seen); the returned tensor is then a view
+        spare page; there is a graph per batch size, bucket of context lengths, class of their mean and reach, captured the second
+        time this key is seen); the returned tensor is then a view
         of the graph's own output buffer and holds its values until the next step of the same size."""
         graph_mode = self._graph_eligible(entries)
         bucket = skew = reach = 0
@@ -319,16 +328,8 @@ class ModelRunner:
         hb = self._prepare(batch, mgr, (bucket + self.block_size - 1) // self.block_size if graph_mode else None,
                            self.graph_batch_size(len(entries)) if graph_mode else 0)
         if places is not None:
-            rows = hb.pinned.numpy()[hb.seg["rows"][0]:]
-            if graph_mode:
-                rows[places] = np.arange(len(places), dtype=np.int32)
-            else:
-                first = np.zeros(len(entries) + 1, dtype=np.int64)             # where each entry's tokens start
-                for at, i in enumerate(places):
-                    first[at + 1] = first[at] + len(entries[i].tokens)
-                start = {i: int(first[at]) for at, i in enumerate(places)}
-                wanted = [start[i] + int(w) for i, e in enumerate(entries) for w in e.want]
-                rows[:len(wanted)] = wanted
+            wanted = self._wanted_rows(entries, places)
+            hb.pinned.numpy()[hb.seg["rows"][0]:][:len(wanted)] = wanted
         self.storage.zero_state_slots(mgr.take_fresh_slots())
         key = (hb.S, bucket, skew, reach) if graph_mode else None
         if graph_mode and (key in self._graphs or key in self._seen_sizes):

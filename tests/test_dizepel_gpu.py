@@ -568,6 +568,28 @@ def test_long_decoding_passes_pages_and_replays_graphs(dtype):
         assert_close({(rid, 2 + i): a for rid in reqs for i, a in enumerate(rows[False][rid])}, ref, dtype, "decode")
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_stand_ins_of_a_replayed_batch_leave_pages_and_states_alone(dtype):
+    """Nine requests on graphs of twelve: the stand-ins' pages and states are their own, so that the steps equal eager ones, which
+    have no stand-ins."""
+    from lmsf_b200.engine.factory import build_model
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    folder, _ = folder_of("X")
+    reqs = requests_for("X", [34 + i for i in range(9)], seed=9)
+    net, _, tdt = build_model(folder, dtype, DEV)
+    rows = {}
+    for eager in (False, True):
+        runner = ModelRunner(net, tdt, torch.device(DEV), 8, num_blocks=64, max_num_seqs=9, enforce_eager=eager)
+        mgr = runner.make_cache_manager()
+        for rid in reqs:
+            mgr.add(rid)
+        runner.step([StepEntry(rid, reqs[rid][:20], []) for rid in reqs], mgr)
+        rows[eager] = [runner.step([StepEntry(rid, [reqs[rid][t]], [0]) for rid in reqs], mgr).float().cpu() for t in range(20, 34)]
+        assert {key[0] for key in runner._graphs} == (set() if eager else {12})
+    for a, b in zip(rows[False], rows[True]):
+        assert float((a - b).abs().max()) <= (1e-5 if dtype == "float32" else 2e-2) * float(b.abs().max())
+
+
 def test_pages_and_slots_of_a_finished_request_serve_the_next():
     """One live request at a time, pages for one and ONE state slot: the second request gets the pages and the states of the
     first, none of which it may see."""

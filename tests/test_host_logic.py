@@ -83,6 +83,48 @@ def test_sizes_of_decode_graphs():
     assert [size(n) for n in (9, 12, 13, 27, 32, 33, 40, 41, 64, 255)] == [12, 12, 16, 28, 32, 40, 40, 48, 64, 256]
 
 
+class _Lengths:
+    """What the order of a batch asks of a cache manager."""
+
+    def __init__(self, cached):
+        self.cached = cached
+
+    def num_tokens(self, rid):
+        return self.cached[rid]
+
+
+def test_requests_that_decode_are_laid_out_longest_first():
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    one = lambda rid, **kw: StepEntry(rid, [7], [0], **kw)
+    order = lambda entries, cached, lens=None, skew=0: ModelRunner._longest_first(entries, _Lengths(cached), lens, skew)
+    # replayed steps: where the class of the graph says that contexts differ; equal lengths keep their order
+    abc = [one("a"), one("b"), one("c"), one("d")]
+    assert order(abc, {}, [5, 90, 5, 91], 1) == [3, 1, 0, 2]
+    assert order(abc, {}, [5, 90, 5, 91], 0) is None and order(abc[:1], {}, [5], 3) is None
+    # other steps: where the longest context is more than a third above the mean; prompt portions come last, in their order
+    mixed = [StepEntry("p", [1, 2, 3], [2]), one("a"), StepEntry("q", [4, 5], []), one("b"), one("c")]
+    assert order(mixed, dict(p=10, a=20, q=900, b=99, c=19)) == [3, 1, 4, 0, 2]
+    assert order(mixed, dict(p=10, a=90, q=900, b=99, c=95)) is None
+    assert order(mixed, dict(p=10, a=2, q=900, b=5, c=5)) is None           # 3, 6 and 6 keys: a fifth above the mean
+    assert order(mixed[:3], dict(p=10, a=20, q=900)) is None                # one request decodes
+    twice = [one("a"), one("b"), one("a")]
+    assert order(twice, dict(a=20, b=99)) is None                           # left to the check that refuses it
+
+
+def test_wanted_rows_follow_the_entries_whatever_the_layout():
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    rng = random.Random(5)
+    for _ in range(200):
+        entries = []
+        for i in range(rng.randint(1, 9)):
+            n = rng.choice([1, 1, 1, 2, 7, 30])
+            entries.append(StepEntry(i, [100 * i + t for t in range(n)], rng.sample(range(n), rng.randint(0, min(n, 4)))))   # any order
+        places = rng.sample(range(len(entries)), len(entries))
+        batch = [t for i in places for t in entries[i].tokens]
+        rows = ModelRunner._wanted_rows(entries, places)
+        assert [batch[r] for r in rows] == [e.tokens[w] for e in entries for w in e.want]
+
+
 def test_token_history_counts_like_a_recount():
     rng = random.Random(0)
     for _ in range(20):

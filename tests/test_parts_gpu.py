@@ -285,9 +285,10 @@ def _register_toy_graph_state():
     register_architecture("ToyGraphStateForTests", dict, spec)
 
 
-def test_a_stateful_mixer_in_replayed_decode_steps_keeps_every_request_state(tmp_path):
-    """Three requests decode together; the batch is padded to four with a stand-in request and replayed from a
-    CUDA graph.  The stand-in's state must go to a slot of its own: each request's logits must equal those it
+@pytest.mark.parametrize("n", [9, 11])
+def test_a_stateful_mixer_in_replayed_decode_steps_keeps_every_request_state(tmp_path, n):
+    """Nine to eleven requests decode together; the batch is padded to twelve with stand-in requests and replayed from a
+    CUDA graph.  The stand-ins' state must go to a slot of its own: each request's logits must equal those it
     gets when it runs alone, step by step, without a graph."""
     from lmsf_b200.engine.factory import build_model
     from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
@@ -296,10 +297,10 @@ def test_a_stateful_mixer_in_replayed_decode_steps_keeps_every_request_state(tmp
                eps=1e-5, max_len=64)
     (tmp_path / "config.json").write_text(json.dumps(cfg))
     model, _, tdt = build_model(str(tmp_path), "float32", DEV, load_format="dummy", seed=5)
-    reqs = {f"s{i}": util.random_ids(14, cfg["vocab"], 70 + i) for i in range(3)}
+    reqs = {f"s{i}": util.random_ids(14, cfg["vocab"], 70 + i) for i in range(n)}
 
     def run(group, enforce_eager):
-        runner = ModelRunner(model, tdt, torch.device(DEV), 8, num_blocks=8, max_num_seqs=4, enforce_eager=enforce_eager)
+        runner = ModelRunner(model, tdt, torch.device(DEV), 8, num_blocks=8, max_num_seqs=12, enforce_eager=enforce_eager)
         mgr = runner.make_cache_manager()
         for rid in group:
             mgr.add(rid)
@@ -311,13 +312,13 @@ def test_a_stateful_mixer_in_replayed_decode_steps_keeps_every_request_state(tmp
             lg = runner.step([StepEntry(rid, [reqs[rid][t]], [0]) for rid in group], mgr)
             for j, rid in enumerate(group):
                 rows[rid].append(lg[j].cpu())
-        replayed = len(runner._graphs)
+        replayed = {key[0] for key in runner._graphs}
         for rid in group:
             mgr.free(rid)
         return rows, replayed
 
     together, replayed = run(list(reqs), enforce_eager=False)
-    assert replayed > 0                           # the steps of three requests ran from a graph of four
+    assert replayed == {12}                       # the steps of all requests ran from graphs of twelve
     for rid in reqs:
         alone, _ = run([rid], enforce_eager=True)
         for a, b in zip(together[rid], alone[rid]):

@@ -138,6 +138,33 @@ def test_one_long_request_decoding_among_short_ones(dtype):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_mixed_steps_of_unequal_contexts_return_their_rows_in_the_order_of_the_entries(dtype):
+    """Decoding requests of 12 to 250 tokens, short ones first, beside prompt portions that want several tokens in any order: the step
+    lays them out longest first, and its logits come back as they were asked for."""
+    from lmsf_b200.engine.model_runner import ModelRunner
+    name, std = "C", 0.15
+    cfg, bs = util.CONFIGS[name], util.BLOCK_SIZE[name]
+    done = [12, 250, 40, 100, 16, 25]                                     # tokens before the mixed step; the third and the last bring portions
+    new = [1, 1, 9, 1, 1, 30]
+    want = [[0], [0], [7, 0, 3], [0], [0], [29, 11]]
+    reqs = {f"u{i}": util.random_ids(d + n, cfg["vocab_size"], 900 + i) for i, (d, n) in enumerate(zip(done, new))}
+    ref = reference(name, dtype, std, reqs)
+    steps = [{"step": 0, "entries": [{"id": rid, "tokens": reqs[rid][:d], "want": []} for rid, d in zip(reqs, done)], "end": []},
+             {"step": 1, "entries": [{"id": rid, "tokens": reqs[rid][d:], "want": w} for rid, d, w in zip(reqs, done, want)], "end": list(reqs)}]
+    laid_out, was = [], ModelRunner._longest_first
+    try:
+        ModelRunner._longest_first = staticmethod(lambda *a: laid_out.append(was(*a)) or laid_out[-1])
+        out = traces.run_inprocess(util.model_folder(name, dtype, std), dtype, steps, bs, traces.max_live_tokens(steps, round_to=bs), max_live=6)
+    finally:
+        ModelRunner._longest_first = staticmethod(was)
+    assert laid_out == [None, [1, 3, 4, 0, 2, 5]]
+    bound, _ = util.logits_bound(dtype, std, ref)
+    rows = traces.collect(steps, out)
+    assert len(rows) == 9
+    assert util.worst_difference(rows, ref) <= bound
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_a_request_dropped_in_the_middle_of_its_prompt_and_replayed(dtype):
     """What preemption by recompute does, at the level of the step function: a live request gives back what it
     holds after 45 of its 130 tokens, its pages go to the others, and it runs again from its first token."""
