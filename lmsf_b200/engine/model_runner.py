@@ -93,9 +93,10 @@ class ModelRunner:
         self.graph_safe = all(getattr(part, "graph_safe", False) for part, _ in model.parts_with_specs())
         self._graphs = OrderedDict()                               # least recently used first
         # Every graph keeps its logits alive.  Together they may hold a 64th of the device's memory (2.8 GB: 86 graphs of 64 requests
-        # and 128,256 logits) and half of what lies free beside the cache and a step's own buffers; then the one unused for longest goes.
-        free, total = torch.cuda.mem_get_info(device)
-        self.graph_output_bytes = max(0, min(total // 64, (free - activation_reserve_bytes) // 2))
+        # and 128,256 logits) and half of what `gpu_memory_utilization` leaves free, or the largest step's alone; then the one unused
+        # for longest goes.  (Reckoned from the device's size: asking what is free would wait for the device.)
+        total = torch.cuda.get_device_properties(device).total_memory
+        self.graph_output_bytes = max(min(total // 64, int(total * (1.0 - gpu_memory_utilization) / 2)), max_num_seqs * self.vocab_size * 4)
         self._seen_sizes = set()
         self._graph_pool = None
         self._capture_stream = None
