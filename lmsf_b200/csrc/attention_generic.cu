@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kWarps * 32) attention_generic_kernel(GenericA
 // value row, then fall on different banks), and asks for the next tile's keys as soon as the scores are made and for its
 // values as soon as these are added up.  Every operation and its order are the kernel's above, to the bit.  What bound that one
 // were the keys, a line of memory per lane and load: a warp spent 4.5 us on a tile with the cache warm.  Four requests of
-// 250 keys, 32 heads of 64: 22.2 -> 7.8 us behind a kernel that has used the L2 up, 10.9 -> 6.9 us else.
+// 250 keys, 32 heads of 64: 22.2 -> 7.8 us behind a kernel that has used the L2 up, 10.9 -> 6.9 us else.  Larger heads stay with the
+// kernel above: at 64 values a block holds 70 KB, three to an SM; at 128 it would hold 135 KB, one to an SM, and that has not been tried.
 __device__ __forceinline__ void cp16(uint32_t dst, const float* src, bool ok) {   // 16 bytes, zeros where there is nothing
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }

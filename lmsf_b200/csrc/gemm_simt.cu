@@ -396,8 +396,10 @@ static int launch_few(const F32Args& a, int batch, cudaStream_t s) {
 }
 
 // At most one block an SM and a long stream each (K of 4,096 and more): the ring takes all of the shared memory.
-// Shorter streams leave room for the next product's blocks, whose first stages then overlap.  (2,048 x 8,192 at 3
-// rows 17.0 -> 14.1 us.)
+// Shorter streams leave room for the next product's blocks, whose first stages then overlap.  (Rings of both depths at 1, 3, 8 and 16
+// rows: 2,048 x 8,192 15.1 -> 13.3, 18.1 -> 13.9, 29.4 -> 22.8 and 58.5 -> 49.6 us; 1,024 x 16,384 28.1 -> 23.2, 31.9 -> 24.5, 55.2 ->
+// 42.5, 112 -> 97; 1,024 x 4,096 7.6 -> 6.6, 8.6 -> 7.0, 14.7 -> 11.6, 28.7 -> 25.0; 256 x 8,192 within 3 %.  Below the line, 2,048 x
+// 2,048: 4.7 -> 4.8, 5.6 -> 5.0, 8.3 -> 7.2, 15.7 -> 13.5 of a product alone after others like it.)
 template <int NT>
 static int launch_few_rows(const F32Args& a, int batch, cudaStream_t s) {
   const bool deep = (long long)ceil_div(a.N, 16) * batch <= sm_count() && a.K >= 4096;
@@ -423,6 +425,10 @@ static int launch_tile(const F32Args& a, int batch, cudaStream_t s) {
   return (int)cudaLaunchKernelEx(&cfg, f32_tile_kernel<CS>, a);
 }
 
+// Few rows: a build takes as many rows as its number says or fewer, and pays for all of them (FMAs, and reads of x from shared
+// memory): 16,384 x 2,048 takes 22.5, 22.4, 23.4, 27.1, 27.3, 34.4 and 61.2 us in the builds of 1, 2, 3, 4, 6, 8 and 16, to a few percent
+// whatever the rows.  So up to 8 rows the builds lie close together, and 5 and 7 rows, which lose little (27.4 and 34.8), go with
+// the next; between 8 and 16 none has been tried.  17 rows by tiles: 123 us.
 static int launch_f32(const F32Args& a, int batch, cudaStream_t s) {
   if (a.M <= 1) return launch_few_rows<1>(a, batch, s);
   if (a.M <= 2) return launch_few_rows<2>(a, batch, s);
@@ -431,10 +437,13 @@ static int launch_f32(const F32Args& a, int batch, cudaStream_t s) {
   if (a.M <= 6) return launch_few_rows<6>(a, batch, s);
   if (a.M <= 8) return launch_few_rows<8>(a, batch, s);
   if (a.M <= 16) return launch_few_rows<16>(a, batch, s);
-  // two blocks fit an SM: the tiles alone where they fill the device, else shared along k
+  // Two blocks fit an SM: the tiles alone where they fill the device, shared by two along k where that fills it, else by eight.  (Alone,
+  // by two, by eight at K = 2,048: 16 tiles 136, 76 and 35 us, 64 tiles 139, 76 and 66, 144 tiles 140, 125 and 133, 216 tiles
+  // 238, 180 and 194, 256 tiles 237, 232 and 226, 1,152 tiles 874, 875 and 960.  Just above a line the sharing below it is still
+  // the better one, because the last wave is nearly empty: 80 tiles 139, 124 and 80, 320 tiles 346, 286 and 279.)
   const long long tiles = (long long)ceil_div(a.M, TM) * ceil_div(a.N, TN) * batch;
-  if (tiles >= 296) return launch_tile<1>(a, batch, s);
-  if (tiles >= 74) return launch_tile<2>(a, batch, s);
+  if (tiles >= 2 * sm_count()) return launch_tile<1>(a, batch, s);
+  if (2 * tiles >= sm_count()) return launch_tile<2>(a, batch, s);
   return launch_tile<8>(a, batch, s);
 }
 

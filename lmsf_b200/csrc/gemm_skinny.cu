@@ -107,8 +107,11 @@ __device__ __forceinline__ void issue_rows(uint32_t stage, const bf16* __restric
 // NT 1 (up to 8 rows): a launch has as many blocks as run at a time, and a block takes several groups of rows in turn, its ring
 // of stages running on from one to the next: the next group's weights are on their way while this one's sums meet and leave.
 // A block of its own for every group stopped its part of the stream from its last stage to its successor's first, about a
-// third of a block's life at K = 2,048.  (One request of the 1B shape 711.6 -> 701.4 us a step, five of the 13B shape 8.22 ->
-// 8.14 ms, the life of five requests of the Dizepel design 9.14 -> 8.78 ms; eight of the 8B shape as before, 3.37 ms.)
+// third of a block's life at K = 2,048.  (This kernel with a group a block and in turn: one request of the 1B shape 767 and 705 us a
+// step, five of the 13B shape 8.24 and 8.05 ms, the life of five requests of the Dizepel design 9.43 and 8.93, eight of the 8B
+// shape 3.33 and 3.28.  The kernel before, which kept its sums where the rings were and had a group a block: 731 where this one
+// takes 718 with the same graphs, and the same for the 13B and 8B shapes.)  9 to 16 rows keep a block a group: their sums still
+// lie where the rings were, and turns have not been tried there.
 template <int NT, int GROUPS, int STAGES, bool ROPE = false, bool PAIR = false>
 __global__ void __launch_bounds__(kWarps * 32) skinny_kernel(Args a) {
   constexpr int kStage = GROUPS * kStageBytes + NT * 8 * kRowBytes;      // W group(s), then x

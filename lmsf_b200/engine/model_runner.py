@@ -226,9 +226,10 @@ class ModelRunner:
     def graph_batch_size(n: int) -> int:
         """Decode batches are replayed from graphs of these sizes: 1 to 8, multiples of 4 up to 32 (where the
         decode attention's plan changes within a few requests: 20 requests take 4.4 ms a step on their own graph and
-        4.7 ms padded to 24), then multiples of 8.  (Few requests, above all of many kv heads, cannot afford stand-ins: 5
-        requests of the 13B shape at 3,900 keys took 8.81 ms a step padded to 8 and take 8.20, because the plan of the attention's splits counted
-        320 pairs of request and head where 200 have keys.)"""
+        4.7 ms padded to 24), then multiples of 8.  (Few requests of many kv heads cannot afford stand-ins: 5
+        requests of the 13B shape at 3,900 keys take 8.76 ms a step padded to 8 and 8.15 as they are, because the plan of the attention's splits
+        counted 320 pairs of request and head where 200 have keys; the life of five requests of the Dizepel design 9.37 and 8.75.  3 and 7
+        requests of the 8B shape, of 8 kv heads, take the same either way: 3.14 and 3.13, 3.05 and 3.04.)"""
         if n <= 8:
             return n
         if n <= 32:
@@ -247,9 +248,10 @@ class ModelRunner:
     @staticmethod
     def graph_reach(bucket: int, max_ctx: int) -> int:
         """The context length that a graph's splits are planned for: its bucket, or in the first bucket 256 or 512 where the
-        longest context is no longer.  (Planned for 1,024 keys, short contexts got splits without keys: the attention of 63
-        requests of 16 to 300 keys took 31.1 us with 2 splits and takes 13.4 with one, of the 1B shape 21.7 with 4 and 8.1 with
-        one, of one request of 97 keys 4.3 and 2.8.)"""
+        longest context is no longer.  (Planned for 1,024 keys, short contexts got splits without keys: a step of 63
+        requests of 16 to 300 keys takes 4.03 ms so and 3.88 with the reach, of the 1B shape 1,091 and 1,038 us, of one request of 97
+        keys 716 and 705; one of the 8B shape at 400 keys 2.85 ms either way.  In later buckets a reach of three quarters made 27
+        requests of the 8B shape at 130 to 2,300 keys slower, 4.53 -> 4.73 ms, and nothing faster.)"""
         r = 256
         while r < max_ctx:
             r *= 2
@@ -321,9 +323,9 @@ class ModelRunner:
         # a graph's block tables are as wide as its bucket of context lengths needs, not as the longest context allowed
         # Requests that decode at unequal lengths are laid out longest first (before the prompt portions), so that the decode
         # attention starts with its longest blocks and the short ones fill its last wave; the rows whose logits are wanted keep
-        # the order of the entries.  (Contexts of 130 to 2,300 tokens: 64 requests of the 1B shape 1,660 -> 1,513 us a step, 27 of
-        # the 8B shape 4,677 -> 4,394, 63 of it beside a portion of 1,985 tokens 31.26 ->
-        # 30.94 ms.)
+        # the order of the entries.  (Contexts of 130 to 2,300 tokens, both orders in turn: 64 requests of the 1B shape 1,630 -> 1,514 us
+        # a step, 27 of the 8B shape 4,674 -> 4,390, 64 of it 6,068 -> 5,510; 17 of the 1B shape 1,125 -> 1,122; 63 of the 8B
+        # shape beside a portion of 1,985 tokens 30.78 -> 30.50 ms, about as much as runs differ.)
         places = self._longest_first(entries, mgr, lens if graph_mode else None, skew)
         batch = entries if places is None else [entries[i] for i in places]
         hb = self._prepare(batch, mgr, (bucket + self.block_size - 1) // self.block_size if graph_mode else None,
