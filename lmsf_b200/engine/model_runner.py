@@ -277,6 +277,8 @@ class ModelRunner:
         """The order in which a step's entries are laid out, or None: as they come.  A replayed step is ordered where its
         graph's class says so; another one where its single tokens' contexts differ (the longest is a third above the mean)."""
         if lens is None:
+            if not all(mgr.has(e.request_id) for e in entries):
+                return None                                    # the checks of the entries, in their order, come first
             lens = [mgr.num_tokens(e.request_id) + 1 if len(e.tokens) == 1 else 0 for e in entries]
             decoding = [n for n in lens if n]
             if len(decoding) < 2 or len(set(e.request_id for e in entries)) < len(entries) or 3 * max(decoding) * len(decoding) <= 4 * sum(decoding):

@@ -92,6 +92,9 @@ class _Lengths:
     def num_tokens(self, rid):
         return self.cached[rid]
 
+    def has(self, rid):
+        return rid in self.cached
+
 
 def test_requests_that_decode_are_laid_out_longest_first():
     from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
@@ -107,8 +110,10 @@ def test_requests_that_decode_are_laid_out_longest_first():
     assert order(mixed, dict(p=10, a=90, q=900, b=99, c=95)) is None
     assert order(mixed, dict(p=10, a=2, q=900, b=5, c=5)) is None           # 3, 6 and 6 keys: a fifth above the mean
     assert order(mixed[:3], dict(p=10, a=20, q=900)) is None                # one request decodes
+    # left to the checks that refuse them, in the order of the entries
+    assert order(mixed, dict(p=10, a=20, q=900, b=99)) is None
     twice = [one("a"), one("b"), one("a")]
-    assert order(twice, dict(a=20, b=99)) is None                           # left to the check that refuses it
+    assert order(twice, dict(a=20, b=99)) is None
 
 
 def test_wanted_rows_follow_the_entries_whatever_the_layout():
