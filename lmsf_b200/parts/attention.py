@@ -396,6 +396,40 @@ def cap_on_tensor_cores(softcap: float, scale: float, kv_planes: int = 2, dist=N
     return not softcap or (scale > 0 and kv_planes == 2 and dist is None and not keep_first and not sigmoid)
 
 
+def decode_lengths(ctx: StepContext, window: Optional[int] = None, keep_first: int = 0, chunk: Optional[int] = None):
+    """(the most keys that a single token of the step sees, the mean): what the decode attention's splits are planned for.  A graph
+    names both itself."""
+    max_ctx, mean_ctx = ctx.extras.get("decode_max_ctx"), ctx.extras.get("decode_mean_ctx")
+    if max_ctx is None or mean_ctx is None:
+        lens = [c for c, n in zip(ctx.ctx_lens, ctx.q_lens) if n == 1]
+        max_ctx = ctx.extras.setdefault("decode_max_ctx", max(lens))
+        mean_ctx = ctx.extras.setdefault("decode_mean_ctx", sum(lens) / len(lens))
+    visible = min(max_ctx, window + (keep_first or 0)) if window else max_ctx
+    if chunk:
+        visible = min(visible, chunk)
+    return visible, min(mean_ctx, visible)
+
+
+def splits_per_request(ctx: StepContext, visible: int, mean_visible: float) -> bool:
+    return SPLITS_PER_REQUEST and ctx.n_decode_seqs >= 2 and mean_visible * 4 <= visible
+
+
+def planned_splits(ctx: StepContext, num_heads: int, num_kv_heads: int, head_dim: int, visible: int, mean_visible: float):
+    # the mean matters to the plan only where it is far below the longest context (a graph names its class)
+    group_size = num_heads // num_kv_heads
+    return kernels.decode_plan(ctx.n_decode_seqs, num_kv_heads, group_size, visible, head_dim, kernels.decode_widths(head_dim, group_size),
+                               mean_ctx=mean_visible if mean_visible * 4 <= visible * 3 else None)
+
+
+def decode_scratch(ctx: StepContext, num_heads: int, splits: int, head_dim: int) -> Optional[torch.Tensor]:
+    """The scratch of the decode attention, one for all layers of a step; None where nothing is split."""
+    need = kernels.attention_decode_scratch_floats(ctx.n_seqs, num_heads, splits, head_dim)
+    scratch = ctx.extras.get("decode_scratch")
+    if need and (scratch is None or scratch.numel() < need):
+        scratch = ctx.extras["decode_scratch"] = torch.zeros(need, dtype=torch.float32, device=ctx.device)
+    return scratch if need else None
+
+
 def paged_attend(ctx: StepContext, out: torch.Tensor, q: torch.Tensor, kv: torch.Tensor, group, *, num_heads: int,
                  num_kv_heads: int, head_dim: int, scale: float, window: Optional[int] = None, softcap: float = 0.0,
                  slopes: Optional[torch.Tensor] = None, kv_planes: int = 2, chunk: Optional[int] = None,
@@ -417,21 +451,10 @@ def paged_attend(ctx: StepContext, out: torch.Tensor, q: torch.Tensor, kv: torch
         extras = dict(chunk=chunk or 0, log_bias=log_bias, sinks=sinks, keep_first=keep_first if window else 0,
                       sigmoid=sigmoid, head_bias=head_bias, dist=dist, softcap=softcap)
         if ctx.n_decode_seqs:
-            max_ctx = ctx.extras.get("decode_max_ctx")
-            if max_ctx is None:
-                max_ctx = ctx.extras["decode_max_ctx"] = max(c for c, n in zip(ctx.ctx_lens, ctx.q_lens) if n == 1)
-            visible = min(max_ctx, window + (keep_first or 0)) if window else max_ctx
-            if chunk:
-                visible = min(visible, chunk)
-            # the mean matters to the plan only where it is far below the longest context (a graph names its class)
-            mean_ctx = ctx.extras.get("decode_mean_ctx")
-            if mean_ctx is None:
-                lens = [c for c, n in zip(ctx.ctx_lens, ctx.q_lens) if n == 1]
-                mean_ctx = ctx.extras["decode_mean_ctx"] = sum(lens) / len(lens)
-            mean_visible = min(mean_ctx, visible)
+            visible, mean_visible = decode_lengths(ctx, window, keep_first, chunk)
             group_size = num_heads // num_kv_heads
             all_decode = ctx.n_decode_seqs == ctx.n_seqs
-            if SPLITS_PER_REQUEST and ctx.n_decode_seqs >= 2 and mean_visible * 4 <= visible:
+            if splits_per_request(ctx, visible, mean_visible):
                 # Requests that differ much in length (a mean of a quarter of the longest and less): splits per
                 # request, from a list of work items that a kernel makes from the step's context lengths (once a
                 # step, for all layers of this geometry).  Measured, 8 layers of the 8B shape: one request at
@@ -460,18 +483,12 @@ def paged_attend(ctx: StepContext, out: torch.Tensor, q: torch.Tensor, kv: torch
                                                num_kv_heads, head_dim, warps, scratch, kv_planes=kv_planes, **extras)
                 splits = None
             else:
-                splits, warps = kernels.decode_plan(ctx.n_decode_seqs, num_kv_heads, group_size, visible,
-                                                    head_dim, kernels.decode_widths(head_dim, group_size),
-                                                    mean_ctx=mean_visible if mean_visible * 4 <= visible * 3 else None)
+                splits, warps = planned_splits(ctx, num_heads, num_kv_heads, head_dim, visible, mean_visible)
             if splits is not None:
-                need = kernels.attention_decode_scratch_floats(ctx.n_seqs, num_heads, splits, head_dim)
-                scratch = ctx.extras.get("decode_scratch")
-                if need and (scratch is None or scratch.numel() < need):
-                    scratch = ctx.extras["decode_scratch"] = torch.zeros(need, dtype=torch.float32, device=q.device)
                 kernels.attention_decode(out, q, kv, group.block_table, group.block_size,
                                          None if all_decode else ctx.decode_seq_ids, ctx.n_decode_seqs, ctx.cu_q,
                                          ctx.ctx_len, scale, window or 0, num_heads,
-                                         num_kv_heads, head_dim, splits, scratch if need else None, warps,
+                                         num_kv_heads, head_dim, splits, decode_scratch(ctx, num_heads, splits, head_dim), warps,
                                          kv_planes=kv_planes, **extras)
         if ctx.n_q_tiles and USE_TC_PREFILL and kernels.tc_attention_supported(q.dtype, head_dim):
             kernels.attention_prefill_tc(out, q, kv, group.block_table, group.block_size, ctx.q_tile128_seq,

@@ -13,6 +13,7 @@ import torch
 
 from .. import kernels
 from ..utils.tracing import span
+from . import plain_layers
 from .base import (Block, KVCacheSpec, LayerCache, ModelSpec, Part, PartSpec, StateSpec, StepContext, build_part,
                    part_class, with_nested)
 
@@ -98,7 +99,11 @@ class DecoderModel:
             x = None
         else:
             x = self.embedding.forward(ctx)
-        for j, call in enumerate(self.calls):
+        # many rows through plain layers: the whole loop in one native call
+        done = plain_layers.run(self, ctx, caches, x) if res is None else None
+        if done is not None:
+            x, res = done
+        for j, call in enumerate(self.calls if done is None else ()):
             block = self.blocks[call.layer]
             if call.entry is not None:
                 if res is None or x is not None:

@@ -1,0 +1,192 @@
+"""The layers of a plain pre-norm decoder in one native call (csrc/plain_layers.cu).
+
+Steps with more rows than the weight-streaming products take (prompts, mixed steps, decode batches above 16) launch nine kernels
+a layer.  Made one by one from Python they cost the host 15 to 20 us each, more than the device needs for them while the rows are
+few.  Where every layer is the plain arrangement (RMSNorm, paged attention with a rotation and without anything a design may add,
+RMSNorm, gated feed-forward; bfloat16; no biases) the loop over them runs in native code, with the same kernels and the same
+arguments.  Anything else keeps the parts' own `forward`.  Whether a model is plain, and where its weights lie, is read anew at
+every step: parts may be changed or given other weights between steps.
+"""
+from __future__ import annotations
+
+import ctypes
+from ctypes import c_float, c_int, c_longlong, c_void_p
+from typing import List, Optional, Tuple
+
+import torch
+
+from .. import kernels
+from ..csrc.build import load_library
+from ..utils import tracing
+from . import attention, linear
+from .attention import PagedAttention
+from .base import LayerCache, StepContext
+from .block import PreNormBlock
+from .mlp import GatedMLP
+from .norm import RMSNorm
+from .rope import RotaryEmbedding
+
+USE_NATIVE_LAYERS = True
+
+
+class _Step(ctypes.Structure):
+    _fields_ = ([(n, c_void_p) for n in ("norm", "rope", "act", "decode", "prefill", "gemm", "get_mode", "set_mode", "handle", "stream",
+                                         "x", "y", "res", "h", "qkv", "att", "gu", "m", "positions", "token_seq", "block_table", "cu_q",
+                                         "ctx_len", "decode_seq_ids", "tile_seq", "tile_q0", "error_flag", "scratch")]
+                + [("page_stride", c_longlong), ("n_pages", c_longlong)]
+                + [(n, c_int) for n in ("tokens", "hidden", "n_q_heads", "n_kv_heads", "head_dim", "ff", "max_blocks", "block_size",
+                                        "n_decode", "n_tiles", "act_code", "n_layers", "n_seqs", "splits", "warps", "pad")])
+
+
+class _Layer(ctypes.Structure):
+    _fields_ = ([(n, c_void_p) for n in ("norm1", "qkv", "o", "norm2", "gate_up", "down", "cache", "inv_freq")]
+                + [(n, c_int) for n in ("norm1_dtype", "norm2_dtype", "rot_dim", "is_neox")]
+                + [(n, c_float) for n in ("eps1", "eps2", "scale")] + [("pad", c_int)])
+
+
+_STAGES = {2: ("rmsnorm.cu", "lmsf_rmsnorm"), 3: ("rope_cache.cu", "lmsf_rope_cache"), 4: ("attention_mma.cu", "lmsf_attention_mma"),
+           5: ("attention_tc.cu", "lmsf_attention_tc"), 6: ("activation.cu", "lmsf_activation")}
+_cublas = None
+
+
+def _library_product():
+    """(cublasGemmEx, cublasGetMathMode, cublasSetMathMode) of the library that torch has loaded, or None."""
+    global _cublas
+    if _cublas is None:
+        try:
+            import os
+            lib = ctypes.CDLL("libcublas.so.12", mode=os.RTLD_NOLOAD | os.RTLD_NOW)
+            _cublas = tuple(ctypes.cast(getattr(lib, n), c_void_p).value
+                            for n in ("cublasGemmEx", "cublasGetMathMode_v2" if hasattr(lib, "cublasGetMathMode_v2") else "cublasGetMathMode",
+                                      "cublasSetMathMode"))
+        except (OSError, AttributeError):
+            _cublas = ()
+    return _cublas or None
+
+
+def _address(source: str, name: str, defines=()) -> int:
+    lib = load_library(source, defines)
+    return ctypes.cast(getattr(lib, name), c_void_p).value
+
+
+_addresses = {}
+
+
+def _entry_points(head_dim: int):
+    a = _addresses.get(head_dim)
+    if a is None:
+        a = _addresses[head_dim] = dict(
+            norm=_address("rmsnorm.cu", "lmsf_add_rmsnorm"), rope=_address("rope_cache.cu", "lmsf_rope_cache_write"),
+            act=_address("activation.cu", "lmsf_gated_act"), decode=_address("attention_mma.cu", "lmsf_attention_decode_width", kernels._mma_defines(head_dim)),
+            prefill=_address("attention_tc.cu", "lmsf_attention_prefill_tc", kernels._mma_defines(head_dim)[:1]))
+        f = load_library("plain_layers.cu").lmsf_plain_layers_run
+        f.restype, f.argtypes = c_int, [c_void_p, c_void_p, c_void_p]
+    return a
+
+
+def plain_attention(m) -> bool:
+    """Whether an attention part is the plain one: rotated queries and keys, a softmax over all keys, nothing beside it."""
+    pe = m.position_encoding
+    return (type(m) is PagedAttention and type(pe) is RotaryEmbedding and pe.mult == 1.0 and m.own_kv and not (
+        m.qk_filter_taps or m.values_are_keys or m.head_gate or m.value_gate or m.qk_norm or m.value_norm or m.has_bias or m.has_out_bias
+        or m.window or m.chunk or m.softcap or m.sigmoid_weights or m.has_head_bias or m.unit_sink or m.learned_sink))
+
+
+def _plain_block(b) -> bool:
+    if type(b) is not PreNormBlock:
+        return False
+    n1, n2, ff = b.mixer_norm, b.ffn_norm, b.feed_forward
+    return (type(n1) is RMSNorm and type(n2) is RMSNorm and not n1.has_layer_scale and not n2.has_layer_scale and type(ff) is GatedMLP
+            and not ff.has_bias and ff.activation in kernels.ACT_CODES and plain_attention(b._mixer))
+
+
+def _matrix(w: Optional[torch.Tensor], rows: int, cols: int) -> int:
+    """The address of a contiguous bfloat16 matrix of this shape on the device, or 0."""
+    if w is None or w.dtype != torch.bfloat16 or not w.is_cuda or w.shape != (rows, cols) or not w.is_contiguous():
+        return 0
+    return w.data_ptr()
+
+
+def _vector(w: Optional[torch.Tensor], n: int) -> Tuple[int, int]:
+    if w is None or not w.is_cuda or w.shape != (n,) or not w.is_contiguous() or w.dtype not in (torch.bfloat16, torch.float32):
+        return 0, 0
+    return w.data_ptr(), kernels.dtype_code(w.dtype)
+
+
+def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
+    """(pending branch, residual stream) behind the last layer, or None where the parts have to run themselves.  x: the embedding."""
+    if not (USE_NATIVE_LAYERS and ctx.dtype == torch.bfloat16 and ctx.n_tokens > kernels.SKINNY_MAX_M and attention.USE_TC_PREFILL
+            and linear.USE_SKINNY and not tracing.ENABLED and model.layer_hook is None and not ctx.extras.get("force_generic_attention")
+            and not torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction):
+        return None
+    calls, blocks = model.calls, model.blocks
+    first = blocks[calls[0].layer] if calls else None
+    if first is None or not _plain_block(first):
+        return None
+    m0, T, D = first._mixer, ctx.n_tokens, first.mixer_norm.hidden_size
+    nh, nkv, hd, ff = m0.num_heads, m0.num_kv_heads, m0.head_dim, first.feed_forward.intermediate_size
+    act, group_index, kv0 = first.feed_forward.activation, caches[0].group, caches[0].kv
+    if hd not in (64, 128) or kv0 is None or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.shape != (T, D) or _library_product() is None:
+        return None
+    group = ctx.groups[group_index]
+    if ctx.n_decode_seqs:
+        visible, mean_visible = attention.decode_lengths(ctx)
+        if attention.splits_per_request(ctx, visible, mean_visible):
+            return None                     # a list of work items that a kernel of the step makes: the parts' own way
+    q_size, kv_size = nh * hd, nkv * hd
+    layers = (_Layer * len(calls))()
+    for j, call in enumerate(calls):
+        b, c = blocks[call.layer], caches[j]
+        if call.entry is not None or call.cache_of is not None or not c.owner or c.group != group_index or c.extra or (j and not _plain_block(b)):
+            return None
+        m, f, n1, n2 = b._mixer, b.feed_forward, b.mixer_norm, b.ffn_norm
+        inv = m.position_encoding.inv_freq
+        if (m.num_heads, m.num_kv_heads, m.head_dim, m.hidden_size, f.intermediate_size, f.activation) != (nh, nkv, hd, D, ff, act) or \
+                c.kv is None or c.kv.shape != kv0.shape or c.kv.dtype != torch.bfloat16 or not c.kv.is_contiguous() or \
+                inv is None or inv.dtype != torch.float32 or inv.numel() * 2 != m.position_encoding.rot_dim:
+            return None
+        l = layers[j]
+        l.qkv, l.o = _matrix(m.qkv, q_size + 2 * kv_size, D), _matrix(m.o, D, q_size)
+        l.gate_up, l.down = _matrix(f.gate_up, 2 * ff, D), _matrix(f.down, D, ff)
+        l.norm1, l.norm1_dtype = _vector(n1.weight, D)
+        l.norm2, l.norm2_dtype = _vector(n2.weight, D)
+        if not (l.qkv and l.o and l.gate_up and l.down and l.norm1 and l.norm2):
+            return None
+        l.cache, l.inv_freq, l.rot_dim, l.is_neox = c.kv.data_ptr(), inv.data_ptr(), m.position_encoding.rot_dim, int(m.position_encoding.is_neox)
+        l.eps1, l.eps2, l.scale = n1.eps, n2.eps, m.scale
+    # The buffers: the pending branch, the normed rows and the residual stream stay; q, k, v and the heads' outputs share their place
+    # with what the feed-forward holds, which is not needed at the same time.
+    up = lambda n: (n + 255) // 256 * 256
+    row, both = up(T * D * 2), max(up(T * (q_size + 2 * kv_size) * 2) + up(T * q_size * 2), up(T * 2 * ff * 2) + up(T * ff * 2))
+    space = torch.empty(row + both, dtype=torch.uint8, device=x.device)
+    y, res = torch.empty_like(x), torch.empty((T, D), dtype=torch.float32, device=x.device)
+    s = _Step(**_entry_points(hd))
+    s.gemm, s.get_mode, s.set_mode = _library_product()
+    s.handle, s.stream = torch.cuda.current_blas_handle(), kernels._stream()
+    at = space.data_ptr()
+    s.x, s.y, s.res, s.h = x.data_ptr(), y.data_ptr(), res.data_ptr(), at
+    s.qkv, s.att = at + row, at + row + up(T * (q_size + 2 * kv_size) * 2)
+    s.gu, s.m = at + row, at + row + up(T * 2 * ff * 2)
+    s.positions, s.token_seq, s.block_table = ctx.positions.data_ptr(), ctx.token_seq.data_ptr(), kernels._i32(group.block_table, "block_table")
+    s.cu_q, s.ctx_len = ctx.cu_q.data_ptr(), ctx.ctx_len.data_ptr()
+    s.max_blocks, s.block_size, s.page_stride, s.n_pages = group.block_table.shape[1], group.block_size, kv0.stride(0), kv0.shape[0]
+    s.error_flag = ctx.error_flag.data_ptr() if ctx.error_flag is not None else None
+    if ctx.n_decode_seqs:
+        s.decode_seq_ids = None if ctx.n_decode_seqs == ctx.n_seqs else ctx.decode_seq_ids.data_ptr()
+        s.splits, s.warps = attention.planned_splits(ctx, nh, nkv, hd, visible, mean_visible)
+        scratch = attention.decode_scratch(ctx, nh, s.splits, hd)
+        s.scratch = scratch.data_ptr() if scratch is not None else None
+    if ctx.n_q_tiles:
+        s.tile_seq, s.tile_q0 = ctx.q_tile128_seq.data_ptr(), ctx.q_tile128_q0.data_ptr()
+    s.n_decode, s.n_tiles = ctx.n_decode_seqs, ctx.n_q_tiles128 if ctx.n_q_tiles else 0
+    s.tokens, s.hidden, s.n_q_heads, s.n_kv_heads, s.head_dim, s.ff = T, D, nh, nkv, hd, ff
+    s.act_code, s.n_layers, s.n_seqs = kernels.ACT_CODES[act], len(calls), ctx.n_seqs
+    rc = c_int(0)
+    n = load_library("plain_layers.cu").lmsf_plain_layers_run(ctypes.byref(s), layers, ctypes.byref(rc))
+    if n < 0:
+        source, prefix = _STAGES.get(-n, (None, None))
+        if source is None:
+            raise kernels.KernelError(f"the library's product failed ({rc.value})")
+        kernels._check(rc.value, source, prefix, kernels._mma_defines(hd) if -n == 4 else kernels._mma_defines(hd)[:1] if -n == 5 else ())
+    kernels.add_launches(n)
+    return y, res

@@ -1,0 +1,84 @@
+"""The layer loop of plain decoders in native code (csrc/plain_layers.cu) against the parts' own forward, to the bit: both make
+the same launches."""
+import pytest
+import torch
+
+import util
+
+pytestmark = pytest.mark.gpu
+
+BASE = dict(architectures=["LlamaForCausalLM"], model_type="llama", hidden_size=256, num_hidden_layers=3, num_attention_heads=4,
+            num_key_value_heads=2, head_dim=64, intermediate_size=448, vocab_size=515, rope_theta=10000.0, rms_norm_eps=1e-5,
+            tie_word_embeddings=False, max_position_embeddings=4096, hidden_act="silu", bos_token_id=1, eos_token_id=2)
+MODELS = {"grouped": BASE, "wide heads": dict(BASE, head_dim=128, num_key_value_heads=4),
+          "scaled": dict(BASE, tie_word_embeddings=True, rope_scaling=dict(rope_type="llama3", factor=8.0, low_freq_factor=1.0,
+                                                                           high_freq_factor=4.0, original_max_position_embeddings=512))}
+
+
+
+
+@pytest.mark.parametrize("name", list(MODELS))
+def test_same_bits_as_the_parts(name, monkeypatch):
+    """Prompts whole and in portions, prompts beside requests that decode, a decode batch above 16, and 16 rows and fewer, which stay with
+    the parts; a model whose second layer is not plain (a window) stays with them whole."""
+    from lmsf_b200.config.registry import resolve_architecture
+    from lmsf_b200 import models  # noqa: F401
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    from lmsf_b200.parts import plain_layers
+    from lmsf_b200.parts.decoder import DecoderModel
+    from lmsf_b200.weights.loader import collect_requirements
+    cfg, dev = dict(MODELS[name]), torch.device("cuda:0")
+    arch = resolve_architecture(cfg)
+    g = torch.Generator(device=dev).manual_seed(5)
+    model = DecoderModel(arch.build_spec(arch.parse_config(cfg)))
+    per_part, parts = {}, {}
+    for part, logical, wspec, names in collect_requirements(model):
+        sizes = [wspec.concrete(i) for i in range(len(wspec.shapes))]
+        shape = (sum(s[0] for s in sizes), *sizes[0][1:])
+        t = torch.randn(shape, generator=g, device=dev) * 0.1 + (1.0 if "norm" in names[0] else 0.0)
+        per_part.setdefault(id(part), {})[logical] = t.to(torch.bfloat16)
+        parts[id(part)] = part
+    for pid, tensors in per_part.items():
+        parts[pid].set_weights(tensors)
+    model.prepare(torch.bfloat16, dev)
+    taken = []
+    inner = plain_layers.run
+
+    def noted(*a):
+        r = inner(*a)
+        taken.append(r is not None)
+        return r
+
+    monkeypatch.setattr(plain_layers, "run", noted)
+    ids = [util.random_ids(n, cfg["vocab_size"], 7 + n) for n in (300, 41, 17, 1)]
+
+    def life(native):
+        monkeypatch.setattr(plain_layers, "USE_NATIVE_LAYERS", native)
+        runner = ModelRunner(model, torch.bfloat16, dev, 16, num_blocks=[300], max_num_seqs=64, max_model_len=1024)
+        mgr = runner.make_cache_manager()
+        out = []
+        step = lambda entries: out.append(runner.step(entries, mgr).clone())
+        for i in range(24):
+            mgr.add(i)
+        step([StepEntry(0, ids[0][:160], [159, 3]), StepEntry(1, ids[1], [40])])                   # prompts
+        step([StepEntry(0, ids[0][160:], [139]), StepEntry(1, [5], [0]), StepEntry(2, ids[2], [16])])   # a later portion, a single token
+        step([StepEntry(2, ids[1][:9], [8])])                                                      # few rows
+        step([StepEntry(i, ids[0][:150], [0]) for i in range(3, 24)])
+        for k in range(3):                                                                         # a decode batch: eager, captured, replayed
+            step([StepEntry(i, [11 + i + k], [0]) for i in range(3, 24)])
+        return out
+
+    taken.clear()
+    a = life(True)
+    assert taken == [True, True, False, True, True, True]          # the last: the capture
+    taken.clear()
+    b = life(False)
+    assert not any(taken)
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+    # one layer that is not plain
+    model.blocks[1]._mixer.window = 50
+    taken.clear()
+    life(True)
+    assert not any(taken)
+    model.blocks[1]._mixer.window = None
