@@ -24,6 +24,7 @@ typedef int (*DecodeFn)(const void*, long long, void*, long long, const void*, l
 typedef int (*PrefillFn)(const void*, long long, long long, void*, long long, const void*, long long, long long, int, int, const int*,
                          int, const int*, const int*, int, const int*, const int*, float, int, int, int, int*, int, int, const float*,
                          const float*, const float*, int, int, const float*, const float*, int, float, void*);
+typedef int (*GatedFn)(void*, long long, const void*, long long, const void*, int, int, int, int, int*, void*);
 typedef cublasStatus_t (*GemmFn)(cublasHandle_t, cublasOperation_t, cublasOperation_t, int, int, int, const void*, const void*,
                                  cudaDataType, int, const void*, cudaDataType, int, const void*, void*, cudaDataType, int,
                                  cublasComputeType_t, cublasGemmAlgo_t);
@@ -34,9 +35,10 @@ typedef cublasStatus_t (*SetModeFn)(cublasHandle_t, cublasMath_t);
 
 struct PlainStep {
   // entry points
-  void *norm, *rope, *act, *decode, *prefill, *gemm, *get_mode, *set_mode, *handle, *stream;
+  void *norm, *rope, *act, *decode, *prefill, *gated, *gemm, *get_mode, *set_mode, *handle, *stream;
   // buffers: x bfloat16 [tokens][hidden] what enters the first layer, y like it the pending branch (out: the last layer's), res
-  // float32 of its shape, h like x, qkv, att [tokens][q width], gu [tokens][2 ff], m [tokens][ff]
+  // float32 of its shape, h like x, qkv, att [tokens][q width], gu [tokens][2 ff] (null: gate, up and activation are one kernel, gemm_gated_tc.cu),
+  // m [tokens][ff]
   void *x, *y, *res, *h, *qkv, *att, *gu, *m;
   // the step's tables
   const int *positions, *token_seq, *block_table, *cu_q, *ctx_len, *decode_seq_ids, *tile_seq, *tile_q0;
@@ -110,10 +112,15 @@ LMSF_API int lmsf_plain_layers_run(const PlainStep* sp, const PlainLayer* layers
     if (!product(s.y, s.att, l.o, D, q_size)) break;
     stage = 2;
     if (!ran(((NormFn)s.norm)(s.h, s.y, (float*)s.res, l.norm2, T, D, l.eps2, 2, LMSF_BF16, l.norm2_dtype, s.stream))) break;
-    stage = 1;
-    if (!product(s.gu, s.h, l.gate_up, 2 * s.ff, D)) break;
-    stage = 6;
-    if (!ran(((ActFn)s.act)(s.m, s.gu, T, s.ff, 2ll * s.ff, s.act_code, LMSF_BF16, s.stream))) break;
+    if (!s.gu) {
+      stage = 7;
+      if (!ran(((GatedFn)s.gated)(s.m, s.ff, s.h, D, l.gate_up, T, s.ff, D, s.act_code, s.error_flag, s.stream))) break;
+    } else {
+      stage = 1;
+      if (!product(s.gu, s.h, l.gate_up, 2 * s.ff, D)) break;
+      stage = 6;
+      if (!ran(((ActFn)s.act)(s.m, s.gu, T, s.ff, 2ll * s.ff, s.act_code, LMSF_BF16, s.stream))) break;
+    }
     stage = 1;
     if (!product(s.y, s.m, l.down, D, s.ff)) break;
     stage = 0;

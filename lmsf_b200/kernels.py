@@ -365,6 +365,48 @@ def gated_act(out: torch.Tensor, x: torch.Tensor, act: str = "silu"):
     _check(rc, "activation.cu", "lmsf_activation")
 
 
+def gemm_gated_tc_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether `gemm_gated_tc` takes x [T, K] and the stacked gate and up rows w [2 I, K]."""
+    return (x.dtype == w.dtype == torch.bfloat16 and x.dim() == w.dim() == 2 and x.shape[1] == w.shape[1] and x.shape[1] % 8 == 0
+            and w.shape[0] % 16 == 0 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_gated_tc(out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, act: str, error_flag: Optional[torch.Tensor] = None):
+    """out[t, i] = act(x[t] . w[i]) * (x[t] . w[I + i]) on tcgen05: both products, in float32, and the activation in one kernel.
+    x: [T, K] rows, w: [2 I, K] contiguous, out: [T, I]; bfloat16."""
+    T, K = x.shape
+    inner = w.shape[0] // 2
+    if not gemm_gated_tc_supported(x, w) or out.shape != (T, inner) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
+        raise KernelError("gemm_gated_tc: x [T, K], w [2 I, K] and out [T, I], bfloat16, with sizes that are multiples of 8")
+    if act not in ACT_CODES:
+        raise KernelError(f"gemm_gated_tc: unknown activation {act!r} (known: {', '.join(sorted(ACT_CODES))})")
+    f = _func("gemm_gated_tc.cu", "lmsf_gemm_gated_tc",
+              [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    rc = f(_ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(w), T, inner, K, ACT_CODES[act],
+           _i32(error_flag if error_flag is not None else error_word(x.device), "error_flag"), _stream())
+    _check(rc, "gemm_gated_tc.cu", "lmsf_gemm_gated_tc")
+
+
+def pairs_fill(rows: int, columns: int, sms: int) -> float:
+    """The share of a launch of gemm_gated_tc that is work: tiles of 256 rows and `columns` tiles of features over sms / 2 pairs of SMs in
+    whole waves, the last block of rows filled as far as it is."""
+    blocks, pairs = -(-rows // 256), max(1, sms // 2)
+    tiles = blocks * columns
+    return rows / (256.0 * blocks) * tiles / (-(-tiles // pairs) * pairs)
+
+
+_SMS = {}
+
+
+def sm_count(device) -> int:
+    key = torch.device(device).index or 0
+    n = _SMS.get(key)
+    if n is None:
+        n = _SMS[key] = torch.cuda.get_device_properties(device).multi_processor_count
+    return n
+
+
 def poly_norm(out: torch.Tensor, x: torch.Tensor, coef: torch.Tensor, eps: float):
     """out[t] = a N(x[t]) + b N(x[t]^2) + c N(x[t]^3) + e with (a, b, c, e) = coef (float32 [4] on the device), powers element
     by element and N the division of a row by its root mean square (eps inside the root); float32 inside.  x: [n, d] view,

@@ -22,6 +22,7 @@ torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 _MM_HAS_OUT_DTYPE: Optional[bool] = None
 USE_SKINNY = True     # bfloat16 products of up to 16 rows run on this package's weight-streaming kernel
+GATED_IN_ONE = True   # gate, up and activation of many rows in one kernel
 SKINNY_TALL_FROM = 65536   # ... except 9 to 16 rows against this many output features and more
 
 
@@ -29,6 +30,14 @@ def _skinny_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
     # (9 to 16 rows against a very tall matrix, the head: a stage of the kernel then holds as much of x as of w, and the
     # library is faster: 162 against 182 us for 128,256 x 4,096 at 16 rows)
     return USE_SKINNY and kernels.gemm_skinny_supported(x, w) and not (x.shape[0] > 8 and w.shape[0] >= SKINNY_TALL_FROM)
+
+
+def gated_in_one(rows: int, width: int, inner: int, device) -> bool:
+    """Whether gate, up and activation run as one kernel (gemm_gated_tc.cu): where its tiles fill their waves.  Where the fill is 0.70 to
+    0.76 (256 and 512 rows of the 8B shape) it takes 56 and 95 us against 64 and 109 of the product and the activation apart; at 0.57
+    (384 rows) 91 against 83.  (Few rows read W at the rate of the memory either way: 0.59 at 200 rows, 54 against 60.)"""
+    return GATED_IN_ONE and width % 8 == 0 and inner % 8 == 0 and \
+        kernels.pairs_fill(rows, -(-inner // 128), kernels.sm_count(device)) >= 0.7
 
 
 def matmul_tn(x: Union[torch.Tensor, Prenormed], w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,

@@ -60,6 +60,13 @@ class GatedMLP(FeedForward):
             kernels.gemm_skinny(m, hx, self.gate_up, fuse_act=self.activation,
                                 prenorm=(h.sumsq, h.eps, h.width) if isinstance(h, Prenormed) else None)
             return self._down(m, then)
+        if not isinstance(h, Prenormed) and self.gate_up_bias is None and self.activation in kernels.ACT_CODES and \
+                kernels.gemm_gated_tc_supported(hx, self.gate_up) and hx.shape[0] > kernels.SKINNY_MAX_M and \
+                linear.gated_in_one(hx.shape[0], hx.shape[1], self.intermediate_size, hx.device):
+            # many rows: gate, up and the activation in one kernel
+            m = torch.empty((hx.shape[0], self.intermediate_size), dtype=hx.dtype, device=hx.device)
+            kernels.gemm_gated_tc(m, hx, self.gate_up, self.activation, ctx.error_flag)
+            return self._down(m, then)
         gu = matmul_tn(h, self.gate_up, bias=self.gate_up_bias)
         m = torch.empty((gu.shape[0], self.intermediate_size), dtype=gu.dtype, device=gu.device)
         if self.activation == "clamped_swiglu":

@@ -30,7 +30,7 @@ USE_NATIVE_LAYERS = True
 
 
 class _Step(ctypes.Structure):
-    _fields_ = ([(n, c_void_p) for n in ("norm", "rope", "act", "decode", "prefill", "gemm", "get_mode", "set_mode", "handle", "stream",
+    _fields_ = ([(n, c_void_p) for n in ("norm", "rope", "act", "decode", "prefill", "gated", "gemm", "get_mode", "set_mode", "handle", "stream",
                                          "x", "y", "res", "h", "qkv", "att", "gu", "m", "positions", "token_seq", "block_table", "cu_q",
                                          "ctx_len", "decode_seq_ids", "tile_seq", "tile_q0", "error_flag", "scratch")]
                 + [("page_stride", c_longlong), ("n_pages", c_longlong)]
@@ -45,7 +45,7 @@ class _Layer(ctypes.Structure):
 
 
 _STAGES = {2: ("rmsnorm.cu", "lmsf_rmsnorm"), 3: ("rope_cache.cu", "lmsf_rope_cache"), 4: ("attention_mma.cu", "lmsf_attention_mma"),
-           5: ("attention_tc.cu", "lmsf_attention_tc"), 6: ("activation.cu", "lmsf_activation")}
+           5: ("attention_tc.cu", "lmsf_attention_tc"), 6: ("activation.cu", "lmsf_activation"), 7: ("gemm_gated_tc.cu", "lmsf_gemm_gated_tc")}
 _cublas = None
 
 
@@ -77,7 +77,7 @@ def _entry_points(head_dim: int):
     if a is None:
         a = _addresses[head_dim] = dict(
             norm=_address("rmsnorm.cu", "lmsf_add_rmsnorm"), rope=_address("rope_cache.cu", "lmsf_rope_cache_write"),
-            act=_address("activation.cu", "lmsf_gated_act"), decode=_address("attention_mma.cu", "lmsf_attention_decode_width", kernels._mma_defines(head_dim)),
+            act=_address("activation.cu", "lmsf_gated_act"), gated=_address("gemm_gated_tc.cu", "lmsf_gemm_gated_tc"), decode=_address("attention_mma.cu", "lmsf_attention_decode_width", kernels._mma_defines(head_dim)),
             prefill=_address("attention_tc.cu", "lmsf_attention_prefill_tc", kernels._mma_defines(head_dim)[:1]))
         f = load_library("plain_layers.cu").lmsf_plain_layers_run
         f.restype, f.argtypes = c_int, [c_void_p, c_void_p, c_void_p]
@@ -157,7 +157,9 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     # The buffers: the pending branch, the normed rows and the residual stream stay; q, k, v and the heads' outputs share their place
     # with what the feed-forward holds, which is not needed at the same time.
     up = lambda n: (n + 255) // 256 * 256
-    row, both = up(T * D * 2), max(up(T * (q_size + 2 * kv_size) * 2) + up(T * q_size * 2), up(T * 2 * ff * 2) + up(T * ff * 2))
+    gated = linear.gated_in_one(T, D, ff, x.device)
+    row, gu_bytes = up(T * D * 2), 0 if gated else up(T * 2 * ff * 2)
+    both = max(up(T * (q_size + 2 * kv_size) * 2) + up(T * q_size * 2), gu_bytes + up(T * ff * 2))
     space = torch.empty(row + both, dtype=torch.uint8, device=x.device)
     y, res = torch.empty_like(x), torch.empty((T, D), dtype=torch.float32, device=x.device)
     s = _Step(**_entry_points(hd))
@@ -166,7 +168,7 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     at = space.data_ptr()
     s.x, s.y, s.res, s.h = x.data_ptr(), y.data_ptr(), res.data_ptr(), at
     s.qkv, s.att = at + row, at + row + up(T * (q_size + 2 * kv_size) * 2)
-    s.gu, s.m = at + row, at + row + up(T * 2 * ff * 2)
+    s.gu, s.m = None if gated else at + row, at + row + gu_bytes
     s.positions, s.token_seq, s.block_table = ctx.positions.data_ptr(), ctx.token_seq.data_ptr(), kernels._i32(group.block_table, "block_table")
     s.cu_q, s.ctx_len = ctx.cu_q.data_ptr(), ctx.ctx_len.data_ptr()
     s.max_blocks, s.block_size, s.page_stride, s.n_pages = group.block_table.shape[1], group.block_size, kv0.stride(0), kv0.shape[0]

@@ -1,0 +1,40 @@
+"""The gate and up products with their activation in one tcgen05 kernel (csrc/gemm_gated_tc.cu), against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("T,I,K", [(1, 8, 8), (17, 128, 64), (128, 136, 72), (129, 120, 200), (256, 1024, 4096), (257, 264, 448),
+                                   (600, 1408, 136), (4500, 512, 512), (9000, 384, 64)])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_gate_and_up_with_their_activation(T, I, K, act):
+    """Edges of the tiles of 256 tokens, 128 features and 64 values of k; more tiles than the device holds pairs; more than one band of
+    tokens; rows of x and of the output longer than what is used.  The result is rounded to bfloat16 once (2^-9 of its value) from float32
+    sums (K 2^-24 of the sums of the terms' absolute values, passed on by at most |u| + |g| each)."""
+    from lmsf_b200 import kernels
+    d = torch.device("cuda:0")
+    g = torch.Generator(device=d).manual_seed(T + I + K)
+    x = torch.randn((T, K + 8), generator=g, device=d).to(torch.bfloat16)[:, :K]
+    w = (torch.randn((2 * I, K), generator=g, device=d) * K ** -0.5).to(torch.bfloat16)
+    out = torch.full((T, I + 8), 7.0, dtype=torch.bfloat16, device=d)
+    flag = torch.zeros(1, dtype=torch.int32, device=d)
+    kernels.gemm_gated_tc(out[:, :I], x, w, act, flag)
+    xd, wd = x.double(), w.double()
+    gate, up = (xd @ wd.T).split(I, 1)
+    a = torch.nn.functional.silu(gate) if act == "silu" else torch.nn.functional.gelu(gate, approximate="tanh")
+    ref = a * up
+    sums = (xd.abs() @ wd.abs().T).split(I, 1)
+    bound = ref.abs() * 2.0 ** -8 + K * 2.0 ** -23 * (sums[0] * up.abs() * 1.2 + sums[1] * a.abs()) + 1e-6
+    assert flag.item() == 0
+    assert ((out[:, :I].double() - ref).abs() <= bound).all()
+    assert (out[:, I:] == 7.0).all()
+
+
+def test_refusals():
+    from lmsf_b200 import kernels
+    z = lambda *s: torch.zeros(s, dtype=torch.bfloat16, device="cuda:0")
+    for x, w, out in ((z(4, 12), z(32, 12), z(4, 16)), (z(4, 16), z(24, 16), z(4, 12)), (z(4, 16), z(32, 16), z(5, 16)),
+                      (z(4, 24)[:, 4:20], z(32, 16), z(4, 16))):
+        with pytest.raises(kernels.KernelError):
+            kernels.gemm_gated_tc(out, x, w, "silu")
