@@ -165,6 +165,10 @@ gated_kernel(const Args a, const __grid_constant__ CUtensorMap x_map, const __gr
         if (++slot == kStages) { slot = 0; ++round; }
       }
     }
+    // The ring once more: the products' arrivals on this CTA's `empty` barriers for the last stages.  The leader's tensor core sends
+    // them here on its own, so neither the last accumulator's arrival nor the cluster's barrier says that they have come, and a CTA
+    // that ends before they do leaves shared memory that is still written.
+    for (int k = max(0, issued - kStages); k < issued && ok; ++k) ok = wait_cluster(empty(k % kStages), (uint32_t)((k / kStages) & 1), failed);
     // after a failure: this CTA's copies land before it ends (the leader's barriers count both CTAs'; the peer's are let land by
     // the wait at the cluster's last barrier, which the leader reaches behind this)
     __syncwarp();

@@ -6,14 +6,17 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,I,K", [(1, 8, 8), (17, 128, 64), (128, 136, 72), (129, 120, 200), (256, 1024, 4096), (257, 264, 448),
-                                   (600, 1408, 136), (4500, 512, 512), (9000, 384, 64)])
+                                   (600, 1408, 136), (4500, 512, 512), (9000, 384, 64), (2100, 6000, 448), (5000, 2568, 840)])
 @pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
 def test_gate_and_up_with_their_activation(T, I, K, act):
-    """Edges of the tiles of 256 tokens, 128 features and 64 values of k; more tiles than the device holds pairs; more than one band of
-    tokens; rows of x and of the output longer than what is used.  The result is rounded to bfloat16 once (2^-9 of its value) from float32
+    """Edges of the tiles of 256 tokens, 128 features and 64 values of k; more than one band of tokens; rows of x and of the output longer
+    than what is used; pairs of CTAs that take five tiles and more in turn, whose accumulators and rings are used again and again (the
+    ring's six stages run on over the edge between two tiles of 7 and of 14 steps, and are awaited once more at the end).  The result is rounded to bfloat16 once (2^-9 of its value) from float32
     sums (K 2^-24 of the sums of the terms' absolute values, passed on by at most |u| + |g| each)."""
     from lmsf_b200 import kernels
     d = torch.device("cuda:0")
+    if T * I > 10 ** 7:
+        assert -(-T // 256) * -(-I // 128) >= 5 * (kernels.sm_count(d) // 2)
     g = torch.Generator(device=d).manual_seed(T + I + K)
     x = torch.randn((T, K + 8), generator=g, device=d).to(torch.bfloat16)[:, :K]
     w = (torch.randn((2 * I, K), generator=g, device=d) * K ** -0.5).to(torch.bfloat16)
