@@ -100,17 +100,41 @@ def _plain_block(b) -> bool:
             and not ff.has_bias and ff.activation in kernels.ACT_CODES and plain_attention(b._mixer))
 
 
-def _matrix(w: Optional[torch.Tensor], rows: int, cols: int) -> int:
+def _matrix(w: Optional[torch.Tensor], rows: int, cols: int, device: torch.device) -> int:
     """The address of a contiguous bfloat16 matrix of this shape on the device, or 0."""
-    if w is None or w.dtype != torch.bfloat16 or not w.is_cuda or w.shape != (rows, cols) or not w.is_contiguous():
+    if w is None or w.dtype != torch.bfloat16 or w.device != device or w.shape != (rows, cols) or not w.is_contiguous():
         return 0
     return w.data_ptr()
 
 
-def _vector(w: Optional[torch.Tensor], n: int) -> Tuple[int, int]:
-    if w is None or not w.is_cuda or w.shape != (n,) or not w.is_contiguous() or w.dtype not in (torch.bfloat16, torch.float32):
+def _vector(w: Optional[torch.Tensor], n: int, device: torch.device) -> Tuple[int, int]:
+    if w is None or w.device != device or w.shape != (n,) or not w.is_contiguous() or w.dtype not in (torch.bfloat16, torch.float32):
         return 0, 0
     return w.data_ptr(), kernels.dtype_code(w.dtype)
+
+
+def _usable(device: torch.device) -> bool:
+    return device.type == "cuda"
+
+
+def _tables_fit(ctx: StepContext, block_table: torch.Tensor, device: torch.device) -> bool:
+    """Whether the step's tables are what the kernels' faces ask for (`kernels._i32`): they go to the native loop as addresses, and
+    nothing behind it can look at them."""
+    tables = [ctx.positions, ctx.token_seq, ctx.cu_q, ctx.ctx_len, block_table]
+    if ctx.error_flag is not None:
+        tables.append(ctx.error_flag)
+    if ctx.n_decode_seqs and ctx.n_decode_seqs != ctx.n_seqs:
+        tables.append(ctx.decode_seq_ids)
+    if ctx.n_q_tiles:
+        tables += [ctx.q_tile128_seq, ctx.q_tile128_q0]
+    return block_table.dim() == 2 and block_table.shape[0] == ctx.n_seqs and all(
+        t is not None and t.dtype == torch.int32 and t.device == device and t.is_contiguous() for t in tables)
+
+
+def _cache_fits(kv: Optional[torch.Tensor], shape: Tuple[int, ...], device: torch.device) -> bool:
+    """Whether a layer's pages are [pages, 2, kv heads, block size, head size] as the step's heads and tables say."""
+    return (kv is not None and kv.dtype == torch.bfloat16 and kv.device == device and tuple(kv.shape) == shape and kv.is_contiguous()
+            and kv.data_ptr() % 16 == 0)
 
 
 def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> Optional[Tuple[torch.Tensor, torch.Tensor]]:
@@ -126,9 +150,15 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     m0, T, D = first._mixer, ctx.n_tokens, first.mixer_norm.hidden_size
     nh, nkv, hd, ff = m0.num_heads, m0.num_kv_heads, m0.head_dim, first.feed_forward.intermediate_size
     act, group_index, kv0 = first.feed_forward.activation, caches[0].group, caches[0].kv
-    if hd not in (64, 128) or kv0 is None or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.shape != (T, D) or _library_product() is None:
+    device = x.device
+    if hd not in (64, 128) or kv0 is None or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.shape != (T, D) or \
+            not _usable(device) or _library_product() is None:
         return None
+    # What the kernels' faces refuse is left to the parts, which say so
     group = ctx.groups[group_index]
+    pages = (kv0.shape[0], 2, nkv, group.block_size, hd)
+    if not _tables_fit(ctx, group.block_table, device):
+        return None
     if ctx.n_decode_seqs:
         visible, mean_visible = attention.decode_lengths(ctx)
         if attention.splits_per_request(ctx, visible, mean_visible):
@@ -142,14 +172,14 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
         m, f, n1, n2 = b._mixer, b.feed_forward, b.mixer_norm, b.ffn_norm
         inv = m.position_encoding.inv_freq
         if (m.num_heads, m.num_kv_heads, m.head_dim, m.hidden_size, f.intermediate_size, f.activation) != (nh, nkv, hd, D, ff, act) or \
-                c.kv is None or c.kv.shape != kv0.shape or c.kv.dtype != torch.bfloat16 or not c.kv.is_contiguous() or \
-                inv is None or inv.dtype != torch.float32 or inv.numel() * 2 != m.position_encoding.rot_dim:
+                not _cache_fits(c.kv, pages, device) or inv is None or inv.dtype != torch.float32 or inv.device != device or \
+                inv.numel() * 2 != m.position_encoding.rot_dim:
             return None
         l = layers[j]
-        l.qkv, l.o = _matrix(m.qkv, q_size + 2 * kv_size, D), _matrix(m.o, D, q_size)
-        l.gate_up, l.down = _matrix(f.gate_up, 2 * ff, D), _matrix(f.down, D, ff)
-        l.norm1, l.norm1_dtype = _vector(n1.weight, D)
-        l.norm2, l.norm2_dtype = _vector(n2.weight, D)
+        l.qkv, l.o = _matrix(m.qkv, q_size + 2 * kv_size, D, device), _matrix(m.o, D, q_size, device)
+        l.gate_up, l.down = _matrix(f.gate_up, 2 * ff, D, device), _matrix(f.down, D, ff, device)
+        l.norm1, l.norm1_dtype = _vector(n1.weight, D, device)
+        l.norm2, l.norm2_dtype = _vector(n2.weight, D, device)
         if not (l.qkv and l.o and l.gate_up and l.down and l.norm1 and l.norm2):
             return None
         l.cache, l.inv_freq, l.rot_dim, l.is_neox = c.kv.data_ptr(), inv.data_ptr(), m.position_encoding.rot_dim, int(m.position_encoding.is_neox)
@@ -157,11 +187,11 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     # The buffers: the pending branch, the normed rows and the residual stream stay; q, k, v and the heads' outputs share their place
     # with what the feed-forward holds, which is not needed at the same time.
     up = lambda n: (n + 255) // 256 * 256
-    gated = linear.gated_in_one(T, D, ff, x.device)
+    gated = linear.gated_in_one(T, D, ff, device)
     row, gu_bytes = up(T * D * 2), 0 if gated else up(T * 2 * ff * 2)
     both = max(up(T * (q_size + 2 * kv_size) * 2) + up(T * q_size * 2), gu_bytes + up(T * ff * 2))
-    space = torch.empty(row + both, dtype=torch.uint8, device=x.device)
-    y, res = torch.empty_like(x), torch.empty((T, D), dtype=torch.float32, device=x.device)
+    space = torch.empty(row + both, dtype=torch.uint8, device=device)
+    y, res = torch.empty_like(x), torch.empty((T, D), dtype=torch.float32, device=device)
     s = _Step(**_entry_points(hd))
     s.gemm, s.get_mode, s.set_mode = _library_product()
     s.handle, s.stream = torch.cuda.current_blas_handle(), kernels._stream()
@@ -169,7 +199,7 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     s.x, s.y, s.res, s.h = x.data_ptr(), y.data_ptr(), res.data_ptr(), at
     s.qkv, s.att = at + row, at + row + up(T * (q_size + 2 * kv_size) * 2)
     s.gu, s.m = None if gated else at + row, at + row + gu_bytes
-    s.positions, s.token_seq, s.block_table = ctx.positions.data_ptr(), ctx.token_seq.data_ptr(), kernels._i32(group.block_table, "block_table")
+    s.positions, s.token_seq, s.block_table = ctx.positions.data_ptr(), ctx.token_seq.data_ptr(), group.block_table.data_ptr()
     s.cu_q, s.ctx_len = ctx.cu_q.data_ptr(), ctx.ctx_len.data_ptr()
     s.max_blocks, s.block_size, s.page_stride, s.n_pages = group.block_table.shape[1], group.block_size, kv0.stride(0), kv0.shape[0]
     s.error_flag = ctx.error_flag.data_ptr() if ctx.error_flag is not None else None

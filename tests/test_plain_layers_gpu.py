@@ -15,19 +15,13 @@ MODELS = {"grouped": BASE, "wide heads": dict(BASE, head_dim=128, num_key_value_
                                                                            high_freq_factor=4.0, original_max_position_embeddings=512))}
 
 
-
-
-@pytest.mark.parametrize("name", list(MODELS))
-def test_same_bits_as_the_parts(name, monkeypatch):
-    """Prompts whole and in portions, prompts beside requests that decode, a decode batch above 16, and 16 rows and fewer, which stay with
-    the parts; a model whose second layer is not plain (a window) stays with them whole."""
+def build(cfg, std=0.1):
+    """A model of random weights on the device, in bfloat16."""
     from lmsf_b200.config.registry import resolve_architecture
     from lmsf_b200 import models  # noqa: F401
-    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
-    from lmsf_b200.parts import plain_layers
     from lmsf_b200.parts.decoder import DecoderModel
     from lmsf_b200.weights.loader import collect_requirements
-    cfg, dev = dict(MODELS[name]), torch.device("cuda:0")
+    cfg, dev = dict(cfg), torch.device("cuda:0")
     arch = resolve_architecture(cfg)
     g = torch.Generator(device=dev).manual_seed(5)
     model = DecoderModel(arch.build_spec(arch.parse_config(cfg)))
@@ -35,12 +29,23 @@ def test_same_bits_as_the_parts(name, monkeypatch):
     for part, logical, wspec, names in collect_requirements(model):
         sizes = [wspec.concrete(i) for i in range(len(wspec.shapes))]
         shape = (sum(s[0] for s in sizes), *sizes[0][1:])
-        t = torch.randn(shape, generator=g, device=dev) * 0.1 + (1.0 if "norm" in names[0] else 0.0)
+        t = torch.randn(shape, generator=g, device=dev) * std + (1.0 if "norm" in names[0] else 0.0)
         per_part.setdefault(id(part), {})[logical] = t.to(torch.bfloat16)
         parts[id(part)] = part
     for pid, tensors in per_part.items():
         parts[pid].set_weights(tensors)
     model.prepare(torch.bfloat16, dev)
+    return model
+
+
+@pytest.mark.parametrize("name", list(MODELS))
+def test_same_bits_as_the_parts(name, monkeypatch):
+    """Prompts whole and in portions, prompts beside requests that decode, a decode batch above 16, and 16 rows and fewer, which stay with
+    the parts; a model whose second layer is not plain (a window) stays with them whole."""
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    from lmsf_b200.parts import plain_layers
+    cfg, dev = MODELS[name], torch.device("cuda:0")
+    model = build(cfg)
     taken = []
     inner = plain_layers.run
 
@@ -82,3 +87,24 @@ def test_same_bits_as_the_parts(name, monkeypatch):
     life(True)
     assert not any(taken)
     model.blocks[1]._mixer.window = None
+
+
+def test_caches_of_another_geometry_are_refused():
+    """Pages of fewer heads or of another size than the step's tables say are refused by the kernels' faces, as without the native loop:
+    it looks at them before it hands their addresses on."""
+    from lmsf_b200 import kernels
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    dev = torch.device("cuda:0")
+    model = build(BASE)
+    runner = ModelRunner(model, torch.bfloat16, dev, 16, num_blocks=[40], max_num_seqs=4, max_model_len=256)
+    mgr = runner.make_cache_manager()
+    mgr.add(0)
+    good = [c.kv for c in runner.storage.layer_caches]
+    for shape in ((41, 2, 1, 16, 64), (41, 2, 2, 8, 64), (41, 1, 2, 16, 64)):
+        for c in runner.storage.layer_caches:
+            c.kv = torch.zeros(shape, dtype=torch.bfloat16, device=dev)
+        with pytest.raises(kernels.KernelError, match="cache of shape"):
+            runner.step([StepEntry(0, util.random_ids(40, BASE["vocab_size"], 1), [39])], mgr)
+    for c, kv in zip(runner.storage.layer_caches, good):
+        c.kv = kv
+    assert torch.isfinite(runner.step([StepEntry(0, util.random_ids(40, BASE["vocab_size"], 1), [39])], mgr)).all()
