@@ -184,10 +184,12 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
             return None
         l.cache, l.inv_freq, l.rot_dim, l.is_neox = c.kv.data_ptr(), inv.data_ptr(), m.position_encoding.rot_dim, int(m.position_encoding.is_neox)
         l.eps1, l.eps2, l.scale = n1.eps, n2.eps, m.scale
+    gated = linear.gated_in_one(T, D, ff, device)
+    if gated and any(l.gate_up % 16 for l in layers):
+        return None                         # the parts choose per layer: the gated kernel wants 16-byte alignment, the library does not
     # The buffers: the pending branch, the normed rows and the residual stream stay; q, k, v and the heads' outputs share their place
     # with what the feed-forward holds, which is not needed at the same time.
     up = lambda n: (n + 255) // 256 * 256
-    gated = linear.gated_in_one(T, D, ff, device)
     row, gu_bytes = up(T * D * 2), 0 if gated else up(T * 2 * ff * 2)
     both = max(up(T * (q_size + 2 * kv_size) * 2) + up(T * q_size * 2), gu_bytes + up(T * ff * 2))
     space = torch.empty(row + both, dtype=torch.uint8, device=device)

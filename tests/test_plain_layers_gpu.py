@@ -108,3 +108,26 @@ def test_caches_of_another_geometry_are_refused():
     for c, kv in zip(runner.storage.layer_caches, good):
         c.kv = kv
     assert torch.isfinite(runner.step([StepEntry(0, util.random_ids(40, BASE["vocab_size"], 1), [39])], mgr)).all()
+
+
+def test_unaligned_weights_are_multiplied_by_the_parts(monkeypatch):
+    """A gate and up matrix at an odd address, in a step whose rows the gated kernel would take: the same logits as from an aligned one but
+    for the rounding of gate and up in one layer of three (2^-9 of the value each; the bound is ten times that)."""
+    from lmsf_b200.engine.model_runner import ModelRunner, StepEntry
+    from lmsf_b200.parts import linear, plain_layers
+    dev = torch.device("cuda:0")
+    model = build(BASE)
+    monkeypatch.setattr(linear, "gated_in_one", lambda *a: True)
+    runner = ModelRunner(model, torch.bfloat16, dev, 16, num_blocks=[40], max_num_seqs=4, max_model_len=256)
+    mgr, ids, out, taken = runner.make_cache_manager(), util.random_ids(100, BASE["vocab_size"], 1), [], []
+    inner = plain_layers.run
+    monkeypatch.setattr(plain_layers, "run", lambda *a: (lambda r: (taken.append(r is not None), r)[1])(inner(*a)))
+    ff = model.blocks[1].feed_forward
+    for i, odd in enumerate((0, 1)):
+        w = torch.empty(ff.gate_up.numel() + odd, dtype=torch.bfloat16, device=dev)[odd:].view(ff.gate_up.shape)
+        w.copy_(ff.gate_up)
+        ff.set_weights({"gate_up": w})
+        mgr.add(i)
+        out.append(runner.step([StepEntry(i, ids, list(range(100)))], mgr).double())
+    assert taken == [True, False]
+    assert (out[0] - out[1]).norm() <= 0.02 * out[0].norm()

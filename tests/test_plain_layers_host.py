@@ -115,3 +115,15 @@ def test_frequencies_elsewhere_are_left_to_the_parts(step):
     pe = step.model.blocks[1]._mixer.position_encoding
     pe.inv_freq = pe.inv_freq.to("meta")
     assert not step.fits() and not step.taken
+
+
+def test_an_unaligned_gate_and_up_matrix_is_left_to_the_parts(step, monkeypatch):
+    """A contiguous matrix at an odd address: the gated kernel would refuse it in the middle of the layers, the parts multiply with the
+    library there.  Without the gated kernel the loop takes it as the library does."""
+    ff = step.model.blocks[1].feed_forward
+    w = ff.gate_up
+    ff.set_weights({"gate_up": torch.zeros(w.numel() + 1, dtype=w.dtype)[1:].view(w.shape)})
+    monkeypatch.setattr(linear, "gated_in_one", lambda *a: True)
+    assert not step.fits() and not step.taken
+    monkeypatch.setattr(linear, "gated_in_one", lambda *a: False)
+    assert step.fits() and step.taken[0]["gu"] is not None
