@@ -185,8 +185,10 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
         l.cache, l.inv_freq, l.rot_dim, l.is_neox = c.kv.data_ptr(), inv.data_ptr(), m.position_encoding.rot_dim, int(m.position_encoding.is_neox)
         l.eps1, l.eps2, l.scale = n1.eps, n2.eps, m.scale
     gated = linear.gated_in_one(T, D, ff, device)
-    if gated and any(l.gate_up % 16 for l in layers):
-        return None                         # the parts choose per layer: the gated kernel wants 16-byte alignment, the library does not
+    if gated and (ctx.error_flag is None or any(l.gate_up % 16 for l in layers)):
+        # The parts' own way: they choose per layer (the gated kernel wants 16-byte alignment, the library does not), and report a wait
+        # that ran out in the device's error word where the step names none
+        return None
     # The buffers: the pending branch, the normed rows and the residual stream stay; q, k, v and the heads' outputs share their place
     # with what the feed-forward holds, which is not needed at the same time.
     up = lambda n: (n + 255) // 256 * 256

@@ -127,3 +127,12 @@ def test_an_unaligned_gate_and_up_matrix_is_left_to_the_parts(step, monkeypatch)
     assert not step.fits() and not step.taken
     monkeypatch.setattr(linear, "gated_in_one", lambda *a: False)
     assert step.fits() and step.taken[0]["gu"] is not None
+
+
+def test_a_step_without_an_error_word_does_not_take_the_gated_kernel_here(step, monkeypatch):
+    """The kernel reports a wait that ran out; its face falls back on the device's own word, which the loop would not."""
+    step.ctx.error_flag = None
+    monkeypatch.setattr(linear, "gated_in_one", lambda *a: True)
+    assert not step.fits() and not step.taken
+    monkeypatch.setattr(linear, "gated_in_one", lambda *a: False)
+    assert step.fits()
