@@ -65,7 +65,7 @@ class GatedMLP(FeedForward):
                 linear.gated_in_one(hx.shape[0], hx.shape[1], self.intermediate_size, hx.device):
             # many rows: gate, up and the activation in one kernel
             m = torch.empty((hx.shape[0], self.intermediate_size), dtype=hx.dtype, device=hx.device)
-            kernels.gemm_gated_tc(m, hx, self.gate_up, self.activation, ctx.error_flag)
+            kernels.gemm_gated_tc(m, hx, self.gate_up, self.activation, ctx.error_flag if ctx is not None else None)
             return self._down(m, then)
         gu = matmul_tn(h, self.gate_up, bias=self.gate_up_bias)
         m = torch.empty((gu.shape[0], self.intermediate_size), dtype=gu.dtype, device=gu.device)
