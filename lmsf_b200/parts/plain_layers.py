@@ -73,12 +73,14 @@ _addresses = {}
 
 
 def _entry_points(head_dim: int):
-    a = _addresses.get(head_dim)
+    defines = kernels._mma_defines(head_dim)              # names the build: a pipeline depth may have been set since the last step
+    a = _addresses.get(defines)
     if a is None:
-        a = _addresses[head_dim] = dict(
+        a = _addresses[defines] = dict(
             norm=_address("rmsnorm.cu", "lmsf_add_rmsnorm"), rope=_address("rope_cache.cu", "lmsf_rope_cache_write"),
-            act=_address("activation.cu", "lmsf_gated_act"), gated=_address("gemm_gated_tc.cu", "lmsf_gemm_gated_tc"), decode=_address("attention_mma.cu", "lmsf_attention_decode_width", kernels._mma_defines(head_dim)),
-            prefill=_address("attention_tc.cu", "lmsf_attention_prefill_tc", kernels._mma_defines(head_dim)[:1]))
+            act=_address("activation.cu", "lmsf_gated_act"), gated=_address("gemm_gated_tc.cu", "lmsf_gemm_gated_tc"),
+            decode=_address("attention_mma.cu", "lmsf_attention_decode_width", defines),
+            prefill=_address("attention_tc.cu", "lmsf_attention_prefill_tc", defines[:1]))
         f = load_library("plain_layers.cu").lmsf_plain_layers_run
         f.restype, f.argtypes = c_int, [c_void_p, c_void_p, c_void_p]
     return a

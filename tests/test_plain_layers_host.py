@@ -136,3 +136,14 @@ def test_a_step_without_an_error_word_does_not_take_the_gated_kernel_here(step, 
     assert not step.fits() and not step.taken
     monkeypatch.setattr(linear, "gated_in_one", lambda *a: False)
     assert step.fits()
+
+
+def test_the_build_of_the_attention_is_the_parts_own(monkeypatch):
+    """A pipeline depth set between two steps names another build of the decode attention, for the loop as for the parts."""
+    monkeypatch.setattr(plain_layers, "_addresses", {})
+    monkeypatch.setattr(plain_layers, "_address", lambda source, name, defines=(): (source, defines))
+    for depth in (None, 2, None):
+        monkeypatch.setattr(kernels, "MMA_KV_STAGES", depth)
+        for head_dim in (64, 128):
+            assert plain_layers._entry_points(head_dim)["decode"] == ("attention_mma.cu", kernels._mma_defines(head_dim))
+            assert plain_layers._entry_points(head_dim)["prefill"] == ("attention_tc.cu", (f"LMSF_HEAD_DIM={head_dim}",))
