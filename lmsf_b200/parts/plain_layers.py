@@ -87,11 +87,13 @@ def _entry_points(head_dim: int):
 
 
 def plain_attention(m) -> bool:
-    """Whether an attention part is the plain one: rotated queries and keys, a softmax over all keys, nothing beside it."""
+    """Whether an attention part is the plain one: rotated queries and keys, a softmax over all keys, nothing beside it (neither
+    declared nor handed over by `set_weights`: the part's own way looks at the tensors)."""
     pe = m.position_encoding
     return (type(m) is PagedAttention and type(pe) is RotaryEmbedding and pe.mult == 1.0 and m.own_kv and not (
         m.qk_filter_taps or m.values_are_keys or m.head_gate or m.value_gate or m.qk_norm or m.value_norm or m.has_bias or m.has_out_bias
-        or m.window or m.chunk or m.softcap or m.sigmoid_weights or m.has_head_bias or m.unit_sink or m.learned_sink))
+        or m.window or m.chunk or m.softcap or m.sigmoid_weights or m.has_head_bias or m.unit_sink or m.learned_sink) and all(
+        t is None for t in (m.qkv_bias, m.o_bias, m._hb32, m._sinks)))
 
 
 def _plain_block(b) -> bool:
@@ -99,7 +101,7 @@ def _plain_block(b) -> bool:
         return False
     n1, n2, ff = b.mixer_norm, b.ffn_norm, b.feed_forward
     return (type(n1) is RMSNorm and type(n2) is RMSNorm and not n1.has_layer_scale and not n2.has_layer_scale and type(ff) is GatedMLP
-            and not ff.has_bias and ff.activation in kernels.ACT_CODES and plain_attention(b._mixer))
+            and not ff.has_bias and ff.gate_up_bias is None and ff.down_bias is None and ff.activation in kernels.ACT_CODES and plain_attention(b._mixer))
 
 
 def _matrix(w: Optional[torch.Tensor], rows: int, cols: int, device: torch.device) -> int:

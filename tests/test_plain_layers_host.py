@@ -147,3 +147,13 @@ def test_the_build_of_the_attention_is_the_parts_own(monkeypatch):
         for head_dim in (64, 128):
             assert plain_layers._entry_points(head_dim)["decode"] == ("attention_mma.cu", kernels._mma_defines(head_dim))
             assert plain_layers._entry_points(head_dim)["prefill"] == ("attention_tc.cu", (f"LMSF_HEAD_DIM={head_dim}",))
+
+
+@pytest.mark.parametrize("part,name,shape,dtype", [("_mixer", "qkv_bias", (512,), torch.bfloat16), ("_mixer", "o_bias", (128,), torch.bfloat16),
+                                                   ("_mixer", "_sinks", (4,), torch.float32), ("_mixer", "_hb32", (4,), torch.float32),
+                                                   ("feed_forward", "gate_up_bias", (512,), torch.bfloat16),
+                                                   ("feed_forward", "down_bias", (128,), torch.bfloat16)])
+def test_biases_that_a_part_was_given_keep_the_parts_own_way(step, part, name, shape, dtype):
+    """A part adds the biases that it holds, whether its parameters spoke of them or not."""
+    getattr(step.model.blocks[1], part).set_weights({name: torch.zeros(shape, dtype=dtype)})
+    assert not step.fits() and not step.taken
