@@ -280,15 +280,12 @@ LMSF_API int lmsf_gemm_gated_tc(void* out, long long ldo, const void* x, long lo
   if ((long long)a.m_tiles * a.f_tiles > (1 << 30)) LMSF_REFUSE("gemm_gated_tc: %d rows are too many", T);
   CUtensorMap xm, wm;
   if (!make_map(&xm, x, T, K, ldx) || !make_map(&wm, W, 2ll * I, K, K)) LMSF_REFUSE("gemm_gated_tc: cuTensorMapEncodeTiled refused the operands' geometry");
-  static int n_sms = 0;
-  if (n_sms == 0) {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 2)
-      LMSF_REFUSE("gemm_gated_tc: the device's number of SMs cannot be read");
-    const cudaError_t e = cudaFuncSetAttribute(gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    n_sms = v;
-  }
+  // asked and set for every call: both belong to the current device, of which a process may use several
+  int dev = 0, n_sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sms < 2)
+    LMSF_REFUSE("gemm_gated_tc: the device's number of SMs cannot be read");
+  const cudaError_t e = cudaFuncSetAttribute(gated_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (e != cudaSuccess) return (int)e;
   const int tiles = a.m_tiles * a.f_tiles, pairs = tiles < n_sms / 2 ? tiles : n_sms / 2;
   return launch_pdl(gated_kernel, dim3(2 * pairs), dim3(kThreads), kSmemBytes, (cudaStream_t)stream, a, xm, wm);
 }
