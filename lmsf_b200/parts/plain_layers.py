@@ -64,6 +64,11 @@ def _library_product():
     return _cublas or None
 
 
+def _products_are_cublas() -> bool:
+    """Whether torch.mm goes to the library that the loop calls (a program may prefer cublasLt for its products)."""
+    return torch.backends.cuda.preferred_blas_library() in (torch._C._BlasBackend.Default, torch._C._BlasBackend.Cublas)
+
+
 def _address(source: str, name: str, defines=()) -> int:
     lib = load_library(source, defines)
     return ctypes.cast(getattr(lib, name), c_void_p).value
@@ -145,7 +150,7 @@ def run(model, ctx: StepContext, caches: List[LayerCache], x: torch.Tensor) -> O
     """(pending branch, residual stream) behind the last layer, or None where the parts have to run themselves.  x: the embedding."""
     if not (USE_NATIVE_LAYERS and ctx.dtype == torch.bfloat16 and ctx.n_tokens > kernels.SKINNY_MAX_M and attention.USE_TC_PREFILL
             and linear.USE_SKINNY and not tracing.ENABLED and model.layer_hook is None and not ctx.extras.get("force_generic_attention")
-            and not torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction):
+            and not torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction and _products_are_cublas()):
         return None
     calls, blocks = model.calls, model.blocks
     first = blocks[calls[0].layer] if calls else None

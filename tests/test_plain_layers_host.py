@@ -157,3 +157,14 @@ def test_biases_that_a_part_was_given_keep_the_parts_own_way(step, part, name, s
     """A part adds the biases that it holds, whether its parameters spoke of them or not."""
     getattr(step.model.blocks[1], part).set_weights({name: torch.zeros(shape, dtype=dtype)})
     assert not step.fits() and not step.taken
+
+
+def test_another_library_for_products_keeps_the_parts_own_way(step):
+    """torch.mm follows a program's choice of library, the loop calls cuBLAS."""
+    before = torch.backends.cuda.preferred_blas_library()
+    try:
+        torch.backends.cuda.preferred_blas_library("cublaslt")
+        assert not step.fits() and not step.taken
+    finally:
+        torch.backends.cuda.preferred_blas_library(before)
+    assert step.fits()
