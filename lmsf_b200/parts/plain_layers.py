@@ -10,6 +10,8 @@ every step: parts may be changed or given other weights between steps.
 from __future__ import annotations
 
 import ctypes
+import os
+import warnings
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import List, Optional, Tuple
 
@@ -50,16 +52,16 @@ _cublas = None
 
 
 def _library_product():
-    """(cublasGemmEx, cublasGetMathMode, cublasSetMathMode) of the library that torch has loaded, or None."""
+    """(cublasGemmEx, cublasGetMathMode, cublasSetMathMode) of the library that torch has loaded, or None (said once)."""
     global _cublas
     if _cublas is None:
+        name = f"libcublas.so.{(torch.version.cuda or '0').split('.')[0]}"
         try:
-            import os
-            lib = ctypes.CDLL("libcublas.so.12", mode=os.RTLD_NOLOAD | os.RTLD_NOW)
-            _cublas = tuple(ctypes.cast(getattr(lib, n), c_void_p).value
-                            for n in ("cublasGemmEx", "cublasGetMathMode_v2" if hasattr(lib, "cublasGetMathMode_v2") else "cublasGetMathMode",
-                                      "cublasSetMathMode"))
-        except (OSError, AttributeError):
+            lib = ctypes.CDLL(name, mode=os.RTLD_NOLOAD | os.RTLD_NOW)
+            _cublas = tuple(ctypes.cast(getattr(lib, n), c_void_p).value for n in ("cublasGemmEx", "cublasGetMathMode", "cublasSetMathMode"))
+        except (OSError, AttributeError) as e:
+            warnings.warn(f"torch's cuBLAS was not found as {name} ({e}); steps of many rows are launched from Python, short prompts take "
+                          f"twice as long", RuntimeWarning, stacklevel=2)
             _cublas = ()
     return _cublas or None
 

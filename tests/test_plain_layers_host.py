@@ -168,3 +168,13 @@ def test_another_library_for_products_keeps_the_parts_own_way(step):
     finally:
         torch.backends.cuda.preferred_blas_library(before)
     assert step.fits()
+
+
+def test_the_library_is_the_one_that_torch_brings(monkeypatch):
+    """It is looked up by torch's own version, and a program is told when it is not there."""
+    monkeypatch.setattr(plain_layers, "_cublas", None)
+    assert len(plain_layers._library_product()) == 3
+    monkeypatch.setattr(plain_layers, "_cublas", None)
+    monkeypatch.setattr(torch.version, "cuda", "99.1")
+    with pytest.warns(RuntimeWarning, match="libcublas.so.99"):
+        assert plain_layers._library_product() is None
