@@ -32,12 +32,29 @@ def _skinny_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
     return USE_SKINNY and kernels.gemm_skinny_supported(x, w) and not (x.shape[0] > 8 and w.shape[0] >= SKINNY_TALL_FROM)
 
 
+def gated_fill_needed(rows: int, width: int) -> float:
+    """How full the gated kernel's waves have to be (`kernels.pairs_fill`) for it to take `rows` rows of a `width`.  What it saves is the
+    activation's pass over memory, which weighs 469 / width of the products; what it loses is the unfilled part of its last wave, where
+    the library has tiles of other sizes to choose from.  So the line rises with the width.  Up to 768 rows and a width of 4,096 it lies at
+    0.70, because the library takes 0.22 to 0.30 us a row there and 0.20 above (28,672 x 4,096).
+    Measured, product and activation apart -> gated, cold weights, us (silu; gelu's tanh form differs by 0 to 7 %, at 0.70 and above
+    it wins wherever silu does; a dozen rows each of 200 to 4,100 a shape):
+    - width 2,048, 8,192 features: fill 0.65 (384 rows) 29.8 -> 30.4, 0.70 (208) 20.8 -> 19.2, 0.69 (1,025) 69.8 -> 69.9, 0.73 (860) 61.9 -> 55.3
+    - 3,072, 8,192: 0.70 (415) 45.1 -> 45.8, 0.76 (450) 48.4 -> 45.0, 0.70 (1,040) 93 -> 102, 0.74 (1,100) 101 -> 104, 0.81 (1,200) 109 -> 103
+    - 4,096, 14,336: 0.57 (384) 90 -> 102, 0.65 (440) 105 -> 105, 0.70 (237) 66 -> 61, 0.70 (474) 113 -> 105, 0.71 (600) 172 -> 132,
+      0.73 (860) 176 -> 187, 0.76 (1,025) 209 -> 215, 0.78 (1,060) 222 -> 215, 0.81 (1,100) 223 -> 214
+    - 5,120, 13,824: 0.72 (380) 102 -> 119, 0.78 (680) 172 -> 182, 0.82 (720) 177 -> 182, 0.83 (1,600) 402 -> 364, 0.89 (470) 128 -> 119
+    - 8,192, 28,672: 0.71 (600) 506 -> 557, 0.81 (1,300) 1,001 -> 1,030, 0.89 (1,200) 917 -> 875
+    (One block of rows reads W at the rate of the memory either way and would gain from 0.6 on at a width of 4,096: 65 -> 60 at 200 rows.)"""
+    if rows <= 768 and width <= 4096:
+        return 0.70
+    return min(0.82, max(0.70, 0.70 + (width - 2048) / 25600.0))
+
+
 def gated_in_one(rows: int, width: int, inner: int, device) -> bool:
-    """Whether gate, up and activation run as one kernel (gemm_gated_tc.cu): where its tiles fill their waves.  Where the fill is 0.70 to
-    0.76 (256 and 512 rows of the 8B shape) it takes 56 and 95 us against 64 and 109 of the product and the activation apart; at 0.57
-    (384 rows) 91 against 83.  (Few rows read W at the rate of the memory either way: 0.59 at 200 rows, 54 against 60.)"""
+    """Whether gate, up and activation run as one kernel (gemm_gated_tc.cu): where its tiles fill their waves (`gated_fill_needed`)."""
     return GATED_IN_ONE and width % 8 == 0 and inner % 8 == 0 and \
-        kernels.pairs_fill(rows, -(-inner // 128), kernels.sm_count(device)) >= 0.7
+        kernels.pairs_fill(rows, -(-inner // 128), kernels.sm_count(device)) >= gated_fill_needed(rows, width)
 
 
 def matmul_tn(x: Union[torch.Tensor, Prenormed], w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
