@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 def test_gate_and_up_with_their_activation(T, I, K, act):
     """Edges of the tiles of 256 tokens, 128 features and 64 values of k; more than one band of tokens; rows of x and of the output longer
     than what is used; pairs of CTAs that take five tiles and more in turn, whose accumulators and rings are used again and again (the
-    ring's six stages run on over the edge between two tiles of 7 and of 14 steps, and are awaited once more at the end).  The result is rounded to bfloat16 once (2^-9 of its value) from float32
-    sums (K 2^-24 of the sums of the terms' absolute values, passed on by at most |u| + |g| each)."""
+    ring's six stages run on over the edge between two tiles of 7 and of 14 steps, and are awaited once more at the end).  The result is rounded to
+    bfloat16 once (2^-8 of its value) from float32 sums, whose partial results the tensor cores may cut off rather than round (K 2^-23 of the
+    sums of the terms' absolute values), passed on by the other factor and by the activation's slope, which is below 1.2."""
     from lmsf_b200 import kernels
     d = torch.device("cuda:0")
     if T * I > 10 ** 7:
@@ -41,3 +42,36 @@ def test_refusals():
                       (z(4, 24)[:, 4:20], z(32, 16), z(4, 16))):
         with pytest.raises(kernels.KernelError):
             kernels.gemm_gated_tc(out, x, w, "silu")
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh"])
+def test_a_row_on_either_side_of_the_choice(act):
+    """The same rows through a feed-forward of 256 rows, whose gate and up stay in float32 up to the activation, and through one of 257, where the
+    library rounds both to bfloat16 first.  A row's result moves with the number of rows beside it, by no more than: gate and up rounded
+    (2^-8 of each, passed on by the other factor and by the activation's slope, below 1.2), their product rounded on both sides, all of it
+    through the down product, and its own rounding on both sides; the down product's float32 sums differ by K 2^-23 of their terms' absolute
+    values, those of gate and up (K 64) by 2^-17, which the factor 1.1 covers."""
+    from lmsf_b200 import kernels
+    from lmsf_b200.parts import linear
+    from lmsf_b200.parts.mlp import GatedMLP
+    d = torch.device("cuda:0")
+    D, inner = 64, kernels.sm_count(d) // 2 * 128
+    assert linear.gated_in_one(256, D, inner, d) and not linear.gated_in_one(257, D, inner, d)
+    g = torch.Generator(device=d).manual_seed(11)
+    w = (torch.randn((2 * inner, D), generator=g, device=d) * D ** -0.5).to(torch.bfloat16)
+    down = (torch.randn((D, inner), generator=g, device=d) * inner ** -0.5).to(torch.bfloat16)
+    x = torch.randn((257, D), generator=g, device=d).to(torch.bfloat16)
+    part = GatedMLP(hidden_size=D, intermediate_size=inner, activation=act)
+    part.set_weights({"gate_up": w, "down": down})
+    one, apart = part.forward(None, x[:256]).double(), part.forward(None, x)[:256].double()
+    xd, u8 = x[:256].double(), 2.0 ** -8
+    gate, up = (xd @ w.double().T).split(inner, 1)
+    a = torch.nn.functional.silu(gate) if act == "silu" else torch.nn.functional.gelu(gate, approximate="tanh")
+    m = (a * up).abs()
+    moved = u8 * (1.2 * gate.abs() * up.abs() + m) + 2 * u8 * m
+    y = (a * up) @ down.double().T
+    bound = 1.1 * (moved @ down.double().abs().T + 2 * u8 * y.abs()) + inner * 2.0 ** -23 * (m @ down.double().abs().T)
+    assert not torch.equal(one, apart)
+    assert ((one - apart).abs() <= bound).all()
+    # and the side that does not round is the nearer one
+    assert (one - y).norm() < (apart - y).norm()
