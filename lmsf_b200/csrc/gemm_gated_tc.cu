@@ -16,9 +16,10 @@
 //              products at K = 2,048: 2,048 x 8,192 116 us, now 91)
 //   warp 8     producer of this CTA's copies
 //   warp 9     issues the products (the leading CTA's alone)
-// Measured, cold weights, product and activation apart -> this kernel: K 4,096, I 14,336: 512 rows 109 -> 95 us, 1,024 204 -> 165,
-// 2,048 372 to 386 -> 302 to 338, 8,192 1,408 to 1,434 -> 1,163 to 1,354 (1.42 to 1.65 PFLOP/s, by the power); K 2,048, I 8,192: 512
-// rows 42 to 55 -> 34, 2,048 116 -> 91, 8,192 464 to 512 -> 355.
+// Measured, cold weights, product and activation apart -> this kernel, by the power that is left to the device: K 4,096, I 14,336: 512
+// rows 108 to 121 -> 95 to 109 us, 1,024 204 to 231 -> 165 to 188, 2,048 361 to 417 -> 302 to 351, 8,192 1,408 to 1,434 -> 1,163 to 1,354 (up
+// to 1.65 PFLOP/s); K 2,048, I 8,192: 512 rows 37 to 39 -> 30 to 32, 2,048 131 to 144 -> 89 to 96, 8,192 464 to 512 -> 355.  At 2,048 x 14,336 the
+// tensor cores are busy in 97 % of the cycles in which an SM works and in 87 % of the launch (the waves are 0.93 full).
 // Every wait is bounded; a block that gives up raises error code 4.
 #include "tc_common.cuh"
 
@@ -85,8 +86,9 @@ __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity, vola
   return done != 0;
 }
 
-// silu by the special-function unit's 2^x and 1/x: within a few 2^-23 times (1 + |g|) of the value, which is rounded to bfloat16
-// next (gate and up are not rounded before, as they are where the activation is a kernel of its own)
+// silu by the special-function unit's 2^x and 1/x: within a few 2^-23 times (1 + |g|) of the value for g above -87.3, which is rounded to
+// bfloat16 next (gate and up are not rounded before, as they are where the activation is a kernel of its own); below, where 1 + e^-g
+// passes 2^126 and its reciprocal is flushed, it is 0 for a value of at most 9e-37 in size
 __device__ __forceinline__ float act_apply(float g, int act) {
   if (act == 0) {
     float e, r;

@@ -3,7 +3,8 @@
 The reference's linear family (core/src/model_executor/layers/linear.rs:28-106, :325-497, :499-728)
 wraps cuBLASLt and merges q, k, v (and gate, up) into one matrix by row ranges; the same merged
 layouts are used here.  bfloat16 products of more than 16 rows go to the library (cuBLAS through torch.mm),
-the place where the reference calls a library too; products of up to 16 rows (decode steps) run on
+the place where the reference calls a library too, but for gate and up where their rows fill the waves of this package's
+tcgen05 kernel (csrc/gemm_gated_tc.cu); products of up to 16 rows (decode steps) run on
 this package's weight-streaming kernel (csrc/gemm_skinny.cu); float32 products run on this package's own FFMA kernel so
 that no reduced-precision mode can slip in and a row's result does not depend on the batch.
 """
@@ -18,6 +19,8 @@ from .base import NormAfter, Part, Prenormed, WeightSpec, register_part
 
 # Library products must add up in float32: with torch's default a split-k bfloat16 product may add its partial sums
 # in bfloat16, and a row's result would then depend on how many rows share the product (on how a prompt was cut).
+# (Two roundings do depend on it: gate and up stay in float32 up to the activation in steps of up to 16 rows and where
+# `gated_in_one` says so, and are rounded to bfloat16 first elsewhere.)
 torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
 
 _MM_HAS_OUT_DTYPE: Optional[bool] = None

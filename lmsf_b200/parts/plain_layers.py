@@ -1,8 +1,9 @@
 """The layers of a plain pre-norm decoder in one native call (csrc/plain_layers.cu).
 
-Steps with more rows than the weight-streaming products take (prompts, mixed steps, decode batches above 16) launch nine kernels
-a layer.  Made one by one from Python they cost the host 15 to 20 us each, more than the device needs for them while the rows are
-few.  Where every layer is the plain arrangement (RMSNorm, paged attention with a rotation and without anything a design may add,
+Steps with more rows than the weight-streaming products take (prompts, mixed steps, decode batches above 16) launch eight to ten
+kernels a layer: four of them products of the library, or three and the gated kernel, and two attentions where prompts run beside
+requests that decode.  Made one by one from Python they cost the host 15 to 20 us each, more than the device needs for them while
+the rows are few.  Where every layer is the plain arrangement (RMSNorm, paged attention with a rotation and without anything a design may add,
 RMSNorm, gated feed-forward; bfloat16; no biases) the loop over them runs in native code, with the same kernels and the same
 arguments.  Anything else keeps the parts' own `forward`.  Whether a model is plain, and where its weights lie, is read anew at
 every step: parts may be changed or given other weights between steps.

@@ -75,3 +75,21 @@ def test_a_row_on_either_side_of_the_choice(act):
     assert ((one - apart).abs() <= bound).all()
     # and the side that does not round is the nearer one
     assert (one - y).norm() < (apart - y).norm()
+
+
+def test_under_capture():
+    """Decode batches large enough for the kernel are replayed from graphs: what a launch asks of the device is allowed while one is recorded."""
+    from lmsf_b200 import kernels
+    d = torch.device("cuda:0")
+    g = torch.Generator(device=d).manual_seed(2)
+    x = torch.randn((260, 192), generator=g, device=d).to(torch.bfloat16)
+    w = torch.randn((2 * 640, 192), generator=g, device=d).to(torch.bfloat16)
+    out, again = (torch.zeros((260, 640), dtype=torch.bfloat16, device=d) for _ in range(2))
+    kernels.gemm_gated_tc(out, x, w, "silu")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        kernels.gemm_gated_tc(again, x, w, "silu")
+    assert not again.any()
+    for _ in range(2):
+        graph.replay()
+    assert torch.equal(out, again)
